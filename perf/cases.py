@@ -201,8 +201,8 @@ def prepare(case, seed):
 
 def _serve_sizes(case):
     """(kind, threads, resolution, spp) of each request of a burst: 60 %
-    renders, 20 % collatz and 20 % fib batches of 2^16 to 2^18 inputs; renders
-    of more than 64 samples x 64^2 pixels are cut to 256^2 at 16."""
+    renders (at most 256^2 pixels at 16 samples, so that the burst stays a
+    short one), 20 % collatz and 20 % fib batches of 2^16 to 2^18 inputs."""
     out = []
     for res, spp, u, lg in _mix(case):
         if u < 0.6:
