@@ -68,6 +68,18 @@ SMALL_REG_VARIANTS = (40, 48)
 LONG_BLOCK_INSTR = 96
 
 
+# Table reads of one block up to this many words above the lowest one of
+# their record share its address (kFlatWords in engine/common.cuh leaves that
+# much room below 2^32).  The path tracer's intersection loop is issue-bound
+# and reads 4 words an iteration, which cost 3 instructions each with an
+# index of their own: 48 batched render requests 19.87 -> 17.53 ms, 320x240x16
+# with default options 3.38 -> 2.97 ms, the 1024x768x64 render 25.94 -> 25.22
+# ms.  One 128-bit load behind a check of the alignment was slower than four
+# words at constant offsets (lane-efficiency form 4.46 against 4.22 ms): the
+# branch pins the loads in a block of their own.
+ROW_SPAN = 63
+
+
 def long_blocks(k: Kernel) -> List[int]:
     """Blocks of at least LONG_BLOCK_INSTR instructions, longest first (at
     most 4)."""
@@ -246,11 +258,82 @@ class Lowering:
             return f"{UNARY_FN[op]}({cv(0, t)})"
         raise NotImplementedError(f"{self.k.name}: op {op}")
 
+    def table_rows(self, instrs):
+        """Table reads of a block that stand at literal distances from one
+        another (a record's fields): every index register is followed through
+        moves and additions of literals, and the reads whose index comes from
+        one value, at most ROW_SPAN words from the lowest, form a row.
+        Returns {position of the row's first read: (index expression of the
+        lowest read, [distances from it])} and {position of a read: (position
+        of its row's first read, distance)}."""
+        origin: Dict[int, tuple] = {}  # register -> (value, distance from it)
+        values = 0
+        reads: Dict[int, List[tuple]] = {}  # value -> [(position, distance)]
+        for pos, ins in enumerate(instrs):
+            if not isinstance(ins, Compute):
+                continue
+            for a in ins.args:
+                if not a.is_literal and a.reg not in origin:
+                    origin[a.reg] = (values, 0)
+                    values += 1
+            a = ins.args[0]
+            if ins.op == "tab" and not a.is_literal and a.type == "u32":
+                v, d = origin[a.reg]
+                reads.setdefault(v, []).append((pos, d))
+            new = (values, 0)
+            if ins.dst.type == "u32" and ins.op == "mov" and not a.is_literal and a.type == "u32":
+                new = origin[a.reg]
+            elif ins.dst.type == "u32" and ins.op == "add" and ins.optype == ("u32",):
+                for x, y in (ins.args, ins.args[::-1]):
+                    if y.is_literal and not x.is_literal and x.type == "u32":
+                        v, d = origin[x.reg]
+                        new = (v, (d + y.bits) & 0xFFFFFFFF)
+                        break
+            if new[0] == values:
+                values += 1
+            origin[ins.dst.reg] = new
+        rows: Dict[int, tuple] = {}
+        member: Dict[int, tuple] = {}
+        for r in reads.values():
+            lo = min(d for _, d in r)
+            r = [(p, d - lo) for p, d in r if d - lo <= ROW_SPAN]
+            dist = sorted({d for _, d in r})
+            if len(dist) < 2:
+                continue
+            first, d0 = r[0]
+            base = self.read(instrs[first].args[0])
+            rows[first] = (base if d0 == 0 else f"{base} - {d0}u", dist)
+            for p, d in r:
+                member[p] = (first, d)
+        return rows, member
+
     def body(self, instrs, indent: str) -> List[str]:
+        rows, member = self.table_rows(instrs)
         out = []
-        for ins in instrs:
-            if isinstance(ins, Compute):
+        for pos, ins in enumerate(instrs):
+            if not isinstance(ins, Compute):
+                continue
+            if pos in rows:
+                base, dist = rows[pos]
+                out.append(indent + f"unsigned {', '.join(f'tw{pos}_{d}' for d in dist)};")
+                out.append(indent + f"const unsigned tb{pos} = static_cast<unsigned>({base});")
+                out.append(indent + "if constexpr(kFlat)")
+                out.append(indent + "{")
+                out.append(indent + f"    const unsigned* tp = ctx.cols->table + tb{pos};")
+                out.extend(indent + f"    tw{pos}_{d} = __ldg(tp + {d});" for d in dist)
+                out.append(indent + "}")
+                out.append(indent + "else")
+                out.append(indent + "{")
+                out.extend(indent + f"    tw{pos}_{d} = table_load<unsigned>(*ctx.cols, tb{pos} + {d}u);" for d in dist)
+                out.append(indent + "}")
+            if pos in member:
+                first, d = member[pos]
+                (t,) = ins.optype
+                out.append(indent + self.write(ins.dst, f"bitcast<{CTYPE[t]}>(tw{first}_{d})"))
+            else:
                 out.append(indent + self.write(ins.dst, self.expr(ins)))
+        if rows:  # a scope of their own: labels of other blocks are jumped to past them
+            out = [indent + "{"] + ["    " + ln for ln in out] + [indent + "}"]
         return out
 
     # ------------------------------------------------------------ transfers
@@ -403,6 +486,10 @@ def generate(k: Kernel) -> str:
     w(f"    static constexpr int kRegroupMaxRegs = {REGROUP_MAX_REGS};")
     # small kernels: two inlined copies of their code in the megakernel
     w(f"    static constexpr bool kSplitCallSites = {'true' if sum(counts) <= REG_VARIANT_MIN_INSTR else 'false'};")
+    # kernels that read records of the table: their launches on flat tables
+    # run instantiations of their own
+    table_rows = any(L.table_rows(b.instrs)[0] for b in k.blocks)
+    w(f"    static constexpr bool kTableRows = {'true' if table_rows else 'false'};")
     w("    struct Regs")
     w("    {")
     for r in regs:
@@ -537,7 +624,8 @@ def generate(k: Kernel) -> str:
     w("    // the warp's vote chose it.  A block that loops on itself takes up")
     w("    // to `spin` further iterations without spending budget (a loop the")
     w("    // warp's lanes run together needs no step of its own per iteration).")
-    w("    template <bool kProf>")
+    w("    // kFlat: the launch's table is flat (Columns::table_flat).")
+    w("    template <bool kProf, bool kFlat>")
     w("    __device__ __forceinline__ static int")
     w("    run_burst(const int entry, Regs& R, Ctx& ctx, unsigned budget, const bool stop_heavy = false,")
     w("              unsigned spin = 0u)")
@@ -788,10 +876,14 @@ def generate(k: Kernel) -> str:
     w("    const unsigned long long grid = (a.n + a.block - 1) / a.block;")
     w("    if(grid == 0) return cudaSuccess;")
     w("    if(a.profile)")
-    w("        plain_kernel<K, true><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(")
+    w("        plain_kernel<K, true, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(")
     w("            a.cols, a.first, a.n, a.max_steps, a.status, a.counters);")
+    if table_rows:
+        w("    else if(!a.cols.table_flat)")
+        w("        plain_kernel<K, false, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(")
+        w("            a.cols, a.first, a.n, a.max_steps, a.status, a.counters);")
     w("    else")
-    w("        plain_kernel<K, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(")
+    w(f"        plain_kernel<K, false, {'true' if table_rows else 'false'}><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(")
     w("            a.cols, a.first, a.n, a.max_steps, a.status, a.counters);")
     w("    return cudaGetLastError();")
     w("}")
@@ -802,11 +894,19 @@ def generate(k: Kernel) -> str:
     w("/// The megakernel at register cap `regs` (0: the default), in its form")
     w("/// for launches that never park when `park` is false; profiled launches")
     w("/// and launches with the staged restore (`bulk`) use the default cap and")
-    w("/// the parking form.  NULL: no such cap compiled.")
-    w("const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park)")
+    w("/// the parking form, and so do launches of a kernel with table records on")
+    w("/// a table that is not flat (the staged-restore instantiation reads")
+    w("/// every word by its own index).  NULL: no such cap compiled.")
+    w("const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park, bool flat)")
     w("{")
     w("    if(profile) return reinterpret_cast<const void*>(&regroup_kernel<K, true, K::kRegroupMaxRegs, true>);")
     w("    if(bulk) return reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, true>);")
+    w("    if(K::kTableRows && !flat)")
+    w("    {")
+    w("        bool known = regs == 0u;")
+    w("        for(const unsigned c: kRegCaps) known |= c == regs;")
+    w("        return known ? reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, true>) : nullptr;")
+    w("    }")
     w("    switch(regs)")
     w("    {")
     w("    case 0u:")
@@ -820,7 +920,7 @@ def generate(k: Kernel) -> str:
     w("cudaError_t launch_regroup(const RegroupLaunch& a)")
     w("{")
     w("    void* args[] = {const_cast<RegroupParams*>(&a.params)};")
-    w("    const void* fn = regroup_fn(a.regs, a.profile, a.params.bulk_restore != 0u, a.park);")
+    w("    const void* fn = regroup_fn(a.regs, a.profile, a.params.bulk_restore != 0u, a.park, a.params.cols.table_flat != 0u);")
     w("    if(!fn) return cudaErrorInvalidValue;")
     w("    if(a.dyn_smem)")
     w("    {")
@@ -833,9 +933,10 @@ def generate(k: Kernel) -> str:
     w("    return cudaLaunchCooperativeKernel(fn, dim3(a.grid), dim3(a.block), args, a.dyn_smem, a.stream);")
     w("}")
     w("")
-    w("cudaError_t regroup_occupancy(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park, int* ctas)")
+    w("cudaError_t regroup_occupancy(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park, bool flat,")
+    w("                              int* ctas)")
     w("{")
-    w("    const void* fn = regroup_fn(regs, profile, dyn_smem != 0u, park);")
+    w("    const void* fn = regroup_fn(regs, profile, dyn_smem != 0u, park, flat);")
     w("    if(!fn) return cudaErrorInvalidValue;")
     w("    if(dyn_smem)")
     w("    {")

@@ -42,7 +42,17 @@ struct Columns
     unsigned long long        ring_mask;
     unsigned long long        tid_base;
     const unsigned*           inst_id;
+    // The table has at most kFlatWords words: the reads of a record (the
+    // fields a block reads at literal distances) then use one address and
+    // constant offsets, one instruction a read instead of three.  0: larger,
+    // or unknown.
+    unsigned                  table_flat;
+    unsigned                  pad0;
 };
+
+/// An index of such a table plus a record's span (below 64) does not wrap in
+/// 32 bits, so word idx + d lies d words above word idx.
+constexpr unsigned long long kFlatWords = 0xffffffffull - 63ull;
 
 /// Position of thread `tid` in the array columns.
 __device__ __forceinline__ unsigned long long

@@ -16,8 +16,9 @@ namespace loom_b200
 /// indexed by the Loom thread id).  Inputs are read once, outputs written
 /// once, registers live in CUDA registers; counters[0..1] receive
 /// thread/warp VM-instruction totals when kProf is set (lane efficiency =
-/// counters[0] / (32 * counters[1])).
-template <typename K, bool kProf>
+/// counters[0] / (32 * counters[1])).  kFlat: the launch's table is flat
+/// (only kernels that read table records have that instantiation).
+template <typename K, bool kProf, bool kFlat>
 __global__ void
 plain_kernel(const Columns                  cols,
              const unsigned long long       first,
@@ -41,7 +42,7 @@ plain_kernel(const Columns                  cols,
         const unsigned budget = max_steps < 0xffffffffull
                                     ? static_cast<unsigned>(max_steps)
                                     : 0xffffffffu;
-        if(K::template run_burst<kProf>(0, R, ctx, budget) != kHalt)
+        if(K::template run_burst<kProf, kFlat>(0, R, ctx, budget) != kHalt)
             ctx.flag(kStatusStepLimit);
         K::store_outputs(R, cols, tid);
     }

@@ -258,6 +258,9 @@ regroup_kernel(const RegroupParams p)
 {
     constexpr int      B    = K::kNumQueues;
     constexpr unsigned FULL = 0xffffffffu;
+    // table records through one address each: every instantiation but the
+    // profiled and the staged-restore one, which serve any table
+    constexpr bool     kFlat = K::kTableRows && !kProf && !kBulk;
     const unsigned lane  = threadIdx.x & 31u;
     const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     __shared__ unsigned long long s_blk[2 * (kProf ? K::kNumBlocks : 1)];
@@ -462,16 +465,16 @@ regroup_kernel(const RegroupParams p)
                             // default (a few iterations let halted lanes take
                             // new threads while the others keep looping)
                             if(minpc && p.spin_iters && p.spin_iters <= 16u)
-                                pc = K::template run_burst<kProf>(pc, R, ctx, 1u, false, 16u);
+                                pc = K::template run_burst<kProf, kFlat>(pc, R, ctx, 1u, false, 16u);
                             else if(minpc && p.spin_iters && p.spin_iters <= 64u)
-                                pc = K::template run_burst<kProf>(pc, R, ctx, 1u, false, 64u);
+                                pc = K::template run_burst<kProf, kFlat>(pc, R, ctx, 1u, false, 64u);
                             else if(minpc)
-                                pc = K::template run_burst<kProf>(pc, R, ctx, 1u, false, kSelfLoopSpin);
+                                pc = K::template run_burst<kProf, kFlat>(pc, R, ctx, 1u, false, kSelfLoopSpin);
                             else
-                                pc = K::template run_burst<kProf>(pc, R, ctx, p.burst, kPark && cost_on && p.schedule < 2u);
+                                pc = K::template run_burst<kProf, kFlat>(pc, R, ctx, p.burst, kPark && cost_on && p.schedule < 2u);
                         }
                         else
-                            pc = K::template run_burst<kProf>(pc, R, ctx, minpc ? 1u : p.burst,
+                            pc = K::template run_burst<kProf, kFlat>(pc, R, ctx, minpc ? 1u : p.burst,
                                                               kPark && cost_on && p.schedule < 2u,
                                                               minpc ? (p.spin_iters ? p.spin_iters : kSelfLoopSpin) : 0u);
                     }

@@ -18,6 +18,7 @@ struct K
     static constexpr int kNumQueues = 1;
     static constexpr int kRegroupMaxRegs = 64;
     static constexpr bool kSplitCallSites = true;
+    static constexpr bool kTableRows = false;
     struct Regs
     {
         unsigned short r0; // a: u16
@@ -101,7 +102,8 @@ struct K
     // the warp's vote chose it.  A block that loops on itself takes up
     // to `spin` further iterations without spending budget (a loop the
     // warp's lanes run together needs no step of its own per iteration).
-    template <bool kProf>
+    // kFlat: the launch's table is flat (Columns::table_flat).
+    template <bool kProf, bool kFlat>
     __device__ __forceinline__ static int
     run_burst(const int entry, Regs& R, Ctx& ctx, unsigned budget, const bool stop_heavy = false,
               unsigned spin = 0u)
@@ -243,10 +245,10 @@ cudaError_t launch_plain(const PlainLaunch& a)
     const unsigned long long grid = (a.n + a.block - 1) / a.block;
     if(grid == 0) return cudaSuccess;
     if(a.profile)
-        plain_kernel<K, true><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
+        plain_kernel<K, true, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
             a.cols, a.first, a.n, a.max_steps, a.status, a.counters);
     else
-        plain_kernel<K, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
+        plain_kernel<K, false, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
             a.cols, a.first, a.n, a.max_steps, a.status, a.counters);
     return cudaGetLastError();
 }
@@ -256,11 +258,19 @@ const unsigned kRegCaps[] = {64u, 40u, 48u};
 /// The megakernel at register cap `regs` (0: the default), in its form
 /// for launches that never park when `park` is false; profiled launches
 /// and launches with the staged restore (`bulk`) use the default cap and
-/// the parking form.  NULL: no such cap compiled.
-const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park)
+/// the parking form, and so do launches of a kernel with table records on
+/// a table that is not flat (the staged-restore instantiation reads
+/// every word by its own index).  NULL: no such cap compiled.
+const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park, bool flat)
 {
     if(profile) return reinterpret_cast<const void*>(&regroup_kernel<K, true, K::kRegroupMaxRegs, true>);
     if(bulk) return reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, true>);
+    if(K::kTableRows && !flat)
+    {
+        bool known = regs == 0u;
+        for(const unsigned c: kRegCaps) known |= c == regs;
+        return known ? reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, true>) : nullptr;
+    }
     switch(regs)
     {
     case 0u:
@@ -277,7 +287,7 @@ const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park)
 cudaError_t launch_regroup(const RegroupLaunch& a)
 {
     void* args[] = {const_cast<RegroupParams*>(&a.params)};
-    const void* fn = regroup_fn(a.regs, a.profile, a.params.bulk_restore != 0u, a.park);
+    const void* fn = regroup_fn(a.regs, a.profile, a.params.bulk_restore != 0u, a.park, a.params.cols.table_flat != 0u);
     if(!fn) return cudaErrorInvalidValue;
     if(a.dyn_smem)
     {
@@ -290,9 +300,10 @@ cudaError_t launch_regroup(const RegroupLaunch& a)
     return cudaLaunchCooperativeKernel(fn, dim3(a.grid), dim3(a.block), args, a.dyn_smem, a.stream);
 }
 
-cudaError_t regroup_occupancy(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park, int* ctas)
+cudaError_t regroup_occupancy(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park, bool flat,
+                              int* ctas)
 {
-    const void* fn = regroup_fn(regs, profile, dyn_smem != 0u, park);
+    const void* fn = regroup_fn(regs, profile, dyn_smem != 0u, park, flat);
     if(!fn) return cudaErrorInvalidValue;
     if(dyn_smem)
     {

@@ -18,6 +18,7 @@ struct K
     static constexpr int kNumQueues = 28;
     static constexpr int kRegroupMaxRegs = 64;
     static constexpr bool kSplitCallSites = false;
+    static constexpr bool kTableRows = true;
     struct Regs
     {
         unsigned int r1; // inst: u32
@@ -260,7 +261,8 @@ struct K
     // the warp's vote chose it.  A block that loops on itself takes up
     // to `spin` further iterations without spending budget (a loop the
     // warp's lanes run together needs no step of its own per iteration).
-    template <bool kProf>
+    // kFlat: the launch's table is flat (Columns::table_flat).
+    template <bool kProf, bool kFlat>
     __device__ __forceinline__ static int
     run_burst(const int entry, Regs& R, Ctx& ctx, unsigned budget, const bool stop_heavy = false,
               unsigned spin = 0u)
@@ -303,37 +305,68 @@ struct K
     L_B0_again:
         fresh = false;
         if constexpr(kProf) count_block(ctx, 0, 32u);
-        R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) * static_cast<unsigned int>(((unsigned int)0x10ull))));
-        R.r7 = static_cast<unsigned int>(table_load<unsigned int>(*ctx.cols, static_cast<unsigned>(R.r6)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-        R.r9 = static_cast<unsigned int>(table_load<unsigned int>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x2ull))));
-        R.r10 = static_cast<unsigned int>(table_load<unsigned int>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x3ull))));
-        R.r11 = static_cast<unsigned int>(table_load<unsigned int>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x4ull))));
-        R.r12 = static_cast<unsigned int>(table_load<unsigned int>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x5ull))));
-        R.r13 = static_cast<unsigned int>(table_load<unsigned int>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x6ull))));
-        R.r14 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x7ull))));
-        R.r15 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x8ull))));
-        R.r16 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x9ull))));
-        R.r17 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r18 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) >> static_cast<unsigned int>(R.r10)));
-        R.r19 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x1ull)) << static_cast<unsigned int>(R.r10)));
-        R.r19 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r19) - static_cast<unsigned int>(((unsigned int)0x1ull))));
-        R.r20 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) & static_cast<unsigned int>(R.r19)));
-        R.r21 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r18) % static_cast<unsigned int>(R.r7)));
-        R.r22 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r18) / static_cast<unsigned int>(R.r7)));
-        R.r23 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r11) ^ static_cast<unsigned int>(((unsigned int)0x1bd11bdaull))));
-        R.r23 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r23) ^ static_cast<unsigned int>(((unsigned int)0x9e3779b9ull))));
-        R.r24 = static_cast<unsigned int>(R.r18);
-        R.r25 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r20) << static_cast<unsigned int>(((unsigned int)0x14ull))));
-        R.r26 = static_cast<unsigned int>(((unsigned int)0x0ull));
+        {
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) * static_cast<unsigned int>(((unsigned int)0x10ull))));
+            unsigned tw1_0, tw1_1, tw1_2, tw1_3, tw1_4, tw1_5, tw1_6, tw1_7, tw1_8, tw1_9;
+            const unsigned tb1 = static_cast<unsigned>(R.r6);
+            if constexpr(kFlat)
+            {
+                const unsigned* tp = ctx.cols->table + tb1;
+                tw1_0 = __ldg(tp + 0);
+                tw1_1 = __ldg(tp + 1);
+                tw1_2 = __ldg(tp + 2);
+                tw1_3 = __ldg(tp + 3);
+                tw1_4 = __ldg(tp + 4);
+                tw1_5 = __ldg(tp + 5);
+                tw1_6 = __ldg(tp + 6);
+                tw1_7 = __ldg(tp + 7);
+                tw1_8 = __ldg(tp + 8);
+                tw1_9 = __ldg(tp + 9);
+            }
+            else
+            {
+                tw1_0 = table_load<unsigned>(*ctx.cols, tb1 + 0u);
+                tw1_1 = table_load<unsigned>(*ctx.cols, tb1 + 1u);
+                tw1_2 = table_load<unsigned>(*ctx.cols, tb1 + 2u);
+                tw1_3 = table_load<unsigned>(*ctx.cols, tb1 + 3u);
+                tw1_4 = table_load<unsigned>(*ctx.cols, tb1 + 4u);
+                tw1_5 = table_load<unsigned>(*ctx.cols, tb1 + 5u);
+                tw1_6 = table_load<unsigned>(*ctx.cols, tb1 + 6u);
+                tw1_7 = table_load<unsigned>(*ctx.cols, tb1 + 7u);
+                tw1_8 = table_load<unsigned>(*ctx.cols, tb1 + 8u);
+                tw1_9 = table_load<unsigned>(*ctx.cols, tb1 + 9u);
+            }
+            R.r7 = static_cast<unsigned int>(bitcast<unsigned int>(tw1_0));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r9 = static_cast<unsigned int>(bitcast<unsigned int>(tw1_1));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x2ull))));
+            R.r10 = static_cast<unsigned int>(bitcast<unsigned int>(tw1_2));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x3ull))));
+            R.r11 = static_cast<unsigned int>(bitcast<unsigned int>(tw1_3));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x4ull))));
+            R.r12 = static_cast<unsigned int>(bitcast<unsigned int>(tw1_4));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x5ull))));
+            R.r13 = static_cast<unsigned int>(bitcast<unsigned int>(tw1_5));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x6ull))));
+            R.r14 = static_cast<float>(bitcast<float>(tw1_6));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x7ull))));
+            R.r15 = static_cast<float>(bitcast<float>(tw1_7));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x8ull))));
+            R.r16 = static_cast<float>(bitcast<float>(tw1_8));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r6) + static_cast<unsigned int>(((unsigned int)0x9ull))));
+            R.r17 = static_cast<float>(bitcast<float>(tw1_9));
+            R.r18 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) >> static_cast<unsigned int>(R.r10)));
+            R.r19 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x1ull)) << static_cast<unsigned int>(R.r10)));
+            R.r19 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r19) - static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r20 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) & static_cast<unsigned int>(R.r19)));
+            R.r21 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r18) % static_cast<unsigned int>(R.r7)));
+            R.r22 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r18) / static_cast<unsigned int>(R.r7)));
+            R.r23 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r11) ^ static_cast<unsigned int>(((unsigned int)0x1bd11bdaull))));
+            R.r23 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r23) ^ static_cast<unsigned int>(((unsigned int)0x9e3779b9ull))));
+            R.r24 = static_cast<unsigned int>(R.r18);
+            R.r25 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r20) << static_cast<unsigned int>(((unsigned int)0x14ull))));
+            R.r26 = static_cast<unsigned int>(((unsigned int)0x0ull));
+        }
         goto L_B23;
     L_B1: // prim
         if(stop_heavy && !fresh) return 1;
@@ -421,43 +454,62 @@ struct K
     L_B3_spin:
         fresh = false;
         if constexpr(kProf) count_block(ctx, 3, 38u);
-        R.r57 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r56)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-        R.r58 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
-        R.r59 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
-        R.r60 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r61 = static_cast<float>(static_cast<float>(static_cast<float>(R.r57) - static_cast<float>(R.r46)));
-        R.r62 = static_cast<float>(static_cast<float>(static_cast<float>(R.r58) - static_cast<float>(R.r47)));
-        R.r63 = static_cast<float>(static_cast<float>(static_cast<float>(R.r59) - static_cast<float>(R.r48)));
-        R.r64 = static_cast<float>((0x0.0p+0f));
-        R.r64 = static_cast<float>(op_fma(R.r61, R.r42, R.r64));
-        R.r64 = static_cast<float>(op_fma(R.r62, R.r43, R.r64));
-        R.r64 = static_cast<float>(op_fma(R.r63, R.r44, R.r64));
-        R.r65 = static_cast<float>(static_cast<float>(-static_cast<float>(R.r64)));
-        R.r66 = static_cast<float>(op_fma(R.r65, R.r42, R.r61));
-        R.r67 = static_cast<float>(op_fma(R.r65, R.r43, R.r62));
-        R.r68 = static_cast<float>(op_fma(R.r65, R.r44, R.r63));
-        R.r69 = static_cast<float>((0x0.0p+0f));
-        R.r69 = static_cast<float>(op_fma(R.r66, R.r66, R.r69));
-        R.r69 = static_cast<float>(op_fma(R.r67, R.r67, R.r69));
-        R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
-        R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
-        R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
-        R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
-        R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
-        R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
-        R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
-        R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
-        R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
-        R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
-        R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
-        R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
-        R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
-        R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-        R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
-        R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
+        {
+            unsigned tw0_0, tw0_1, tw0_2, tw0_3;
+            const unsigned tb0 = static_cast<unsigned>(R.r56);
+            if constexpr(kFlat)
+            {
+                const unsigned* tp = ctx.cols->table + tb0;
+                tw0_0 = __ldg(tp + 0);
+                tw0_1 = __ldg(tp + 1);
+                tw0_2 = __ldg(tp + 2);
+                tw0_3 = __ldg(tp + 3);
+            }
+            else
+            {
+                tw0_0 = table_load<unsigned>(*ctx.cols, tb0 + 0u);
+                tw0_1 = table_load<unsigned>(*ctx.cols, tb0 + 1u);
+                tw0_2 = table_load<unsigned>(*ctx.cols, tb0 + 2u);
+                tw0_3 = table_load<unsigned>(*ctx.cols, tb0 + 3u);
+            }
+            R.r57 = static_cast<float>(bitcast<float>(tw0_0));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r58 = static_cast<float>(bitcast<float>(tw0_1));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
+            R.r59 = static_cast<float>(bitcast<float>(tw0_2));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
+            R.r60 = static_cast<float>(bitcast<float>(tw0_3));
+            R.r61 = static_cast<float>(static_cast<float>(static_cast<float>(R.r57) - static_cast<float>(R.r46)));
+            R.r62 = static_cast<float>(static_cast<float>(static_cast<float>(R.r58) - static_cast<float>(R.r47)));
+            R.r63 = static_cast<float>(static_cast<float>(static_cast<float>(R.r59) - static_cast<float>(R.r48)));
+            R.r64 = static_cast<float>((0x0.0p+0f));
+            R.r64 = static_cast<float>(op_fma(R.r61, R.r42, R.r64));
+            R.r64 = static_cast<float>(op_fma(R.r62, R.r43, R.r64));
+            R.r64 = static_cast<float>(op_fma(R.r63, R.r44, R.r64));
+            R.r65 = static_cast<float>(static_cast<float>(-static_cast<float>(R.r64)));
+            R.r66 = static_cast<float>(op_fma(R.r65, R.r42, R.r61));
+            R.r67 = static_cast<float>(op_fma(R.r65, R.r43, R.r62));
+            R.r68 = static_cast<float>(op_fma(R.r65, R.r44, R.r63));
+            R.r69 = static_cast<float>((0x0.0p+0f));
+            R.r69 = static_cast<float>(op_fma(R.r66, R.r66, R.r69));
+            R.r69 = static_cast<float>(op_fma(R.r67, R.r67, R.r69));
+            R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
+            R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
+            R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
+            R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
+            R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
+            R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
+            R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
+            R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
+            R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
+            R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
+            R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
+            R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
+            R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+            R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
+            R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
+        }
         if(R.r33) { if(spin != 0u) { --spin; goto L_B3_spin; } goto L_B3_again; } else goto L_B4;
     L_B4: // shade
         fresh = false;
@@ -469,33 +521,60 @@ struct K
     L_B5_again:
         fresh = false;
         if constexpr(kProf) count_block(ctx, 5, 28u);
-        R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r54) * static_cast<unsigned int>(((unsigned int)0x8ull))));
-        R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(R.r12)));
-        R.r57 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r56)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-        R.r58 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
-        R.r59 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
-        R.r60 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x4ull))));
-        R.r76 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x5ull))));
-        R.r77 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x6ull))));
-        R.r78 = static_cast<float>(table_load<float>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x7ull))));
-        R.r79 = static_cast<unsigned int>(table_load<unsigned int>(*ctx.cols, static_cast<unsigned>(R.r8)));
-        R.r80 = static_cast<float>(op_fma(R.r42, R.r53, R.r46));
-        R.r81 = static_cast<float>(op_fma(R.r43, R.r53, R.r47));
-        R.r82 = static_cast<float>(op_fma(R.r44, R.r53, R.r48));
-        R.r83 = static_cast<float>(static_cast<float>(static_cast<float>(R.r80) - static_cast<float>(R.r57)));
-        R.r84 = static_cast<float>(static_cast<float>(static_cast<float>(R.r81) - static_cast<float>(R.r58)));
-        R.r85 = static_cast<float>(static_cast<float>(static_cast<float>(R.r82) - static_cast<float>(R.r59)));
-        R.r83 = static_cast<float>(static_cast<float>(static_cast<float>(R.r83) / static_cast<float>(R.r60)));
-        R.r84 = static_cast<float>(static_cast<float>(static_cast<float>(R.r84) / static_cast<float>(R.r60)));
-        R.r85 = static_cast<float>(static_cast<float>(static_cast<float>(R.r85) / static_cast<float>(R.r60)));
-        R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r79) == static_cast<unsigned int>(((unsigned int)0x3ull))));
+        {
+            R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r54) * static_cast<unsigned int>(((unsigned int)0x8ull))));
+            R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(R.r12)));
+            unsigned tw2_0, tw2_1, tw2_2, tw2_3, tw2_4, tw2_5, tw2_6, tw2_7;
+            const unsigned tb2 = static_cast<unsigned>(R.r56);
+            if constexpr(kFlat)
+            {
+                const unsigned* tp = ctx.cols->table + tb2;
+                tw2_0 = __ldg(tp + 0);
+                tw2_1 = __ldg(tp + 1);
+                tw2_2 = __ldg(tp + 2);
+                tw2_3 = __ldg(tp + 3);
+                tw2_4 = __ldg(tp + 4);
+                tw2_5 = __ldg(tp + 5);
+                tw2_6 = __ldg(tp + 6);
+                tw2_7 = __ldg(tp + 7);
+            }
+            else
+            {
+                tw2_0 = table_load<unsigned>(*ctx.cols, tb2 + 0u);
+                tw2_1 = table_load<unsigned>(*ctx.cols, tb2 + 1u);
+                tw2_2 = table_load<unsigned>(*ctx.cols, tb2 + 2u);
+                tw2_3 = table_load<unsigned>(*ctx.cols, tb2 + 3u);
+                tw2_4 = table_load<unsigned>(*ctx.cols, tb2 + 4u);
+                tw2_5 = table_load<unsigned>(*ctx.cols, tb2 + 5u);
+                tw2_6 = table_load<unsigned>(*ctx.cols, tb2 + 6u);
+                tw2_7 = table_load<unsigned>(*ctx.cols, tb2 + 7u);
+            }
+            R.r57 = static_cast<float>(bitcast<float>(tw2_0));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r58 = static_cast<float>(bitcast<float>(tw2_1));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
+            R.r59 = static_cast<float>(bitcast<float>(tw2_2));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
+            R.r60 = static_cast<float>(bitcast<float>(tw2_3));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x4ull))));
+            R.r76 = static_cast<float>(bitcast<float>(tw2_4));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x5ull))));
+            R.r77 = static_cast<float>(bitcast<float>(tw2_5));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x6ull))));
+            R.r78 = static_cast<float>(bitcast<float>(tw2_6));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x7ull))));
+            R.r79 = static_cast<unsigned int>(bitcast<unsigned int>(tw2_7));
+            R.r80 = static_cast<float>(op_fma(R.r42, R.r53, R.r46));
+            R.r81 = static_cast<float>(op_fma(R.r43, R.r53, R.r47));
+            R.r82 = static_cast<float>(op_fma(R.r44, R.r53, R.r48));
+            R.r83 = static_cast<float>(static_cast<float>(static_cast<float>(R.r80) - static_cast<float>(R.r57)));
+            R.r84 = static_cast<float>(static_cast<float>(static_cast<float>(R.r81) - static_cast<float>(R.r58)));
+            R.r85 = static_cast<float>(static_cast<float>(static_cast<float>(R.r82) - static_cast<float>(R.r59)));
+            R.r83 = static_cast<float>(static_cast<float>(static_cast<float>(R.r83) / static_cast<float>(R.r60)));
+            R.r84 = static_cast<float>(static_cast<float>(static_cast<float>(R.r84) / static_cast<float>(R.r60)));
+            R.r85 = static_cast<float>(static_cast<float>(static_cast<float>(R.r85) / static_cast<float>(R.r60)));
+            R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r79) == static_cast<unsigned int>(((unsigned int)0x3ull))));
+        }
         if(R.r33) goto L_B6; else goto L_B7;
     L_B6: // emit
         fresh = false;
@@ -5074,10 +5153,13 @@ cudaError_t launch_plain(const PlainLaunch& a)
     const unsigned long long grid = (a.n + a.block - 1) / a.block;
     if(grid == 0) return cudaSuccess;
     if(a.profile)
-        plain_kernel<K, true><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
+        plain_kernel<K, true, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
+            a.cols, a.first, a.n, a.max_steps, a.status, a.counters);
+    else if(!a.cols.table_flat)
+        plain_kernel<K, false, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
             a.cols, a.first, a.n, a.max_steps, a.status, a.counters);
     else
-        plain_kernel<K, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
+        plain_kernel<K, false, true><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
             a.cols, a.first, a.n, a.max_steps, a.status, a.counters);
     return cudaGetLastError();
 }
@@ -5087,11 +5169,19 @@ const unsigned kRegCaps[] = {64u, 32u, 40u, 48u, 56u, 80u, 96u, 128u};
 /// The megakernel at register cap `regs` (0: the default), in its form
 /// for launches that never park when `park` is false; profiled launches
 /// and launches with the staged restore (`bulk`) use the default cap and
-/// the parking form.  NULL: no such cap compiled.
-const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park)
+/// the parking form, and so do launches of a kernel with table records on
+/// a table that is not flat (the staged-restore instantiation reads
+/// every word by its own index).  NULL: no such cap compiled.
+const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park, bool flat)
 {
     if(profile) return reinterpret_cast<const void*>(&regroup_kernel<K, true, K::kRegroupMaxRegs, true>);
     if(bulk) return reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, true>);
+    if(K::kTableRows && !flat)
+    {
+        bool known = regs == 0u;
+        for(const unsigned c: kRegCaps) known |= c == regs;
+        return known ? reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, true>) : nullptr;
+    }
     switch(regs)
     {
     case 0u:
@@ -5118,7 +5208,7 @@ const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park)
 cudaError_t launch_regroup(const RegroupLaunch& a)
 {
     void* args[] = {const_cast<RegroupParams*>(&a.params)};
-    const void* fn = regroup_fn(a.regs, a.profile, a.params.bulk_restore != 0u, a.park);
+    const void* fn = regroup_fn(a.regs, a.profile, a.params.bulk_restore != 0u, a.park, a.params.cols.table_flat != 0u);
     if(!fn) return cudaErrorInvalidValue;
     if(a.dyn_smem)
     {
@@ -5131,9 +5221,10 @@ cudaError_t launch_regroup(const RegroupLaunch& a)
     return cudaLaunchCooperativeKernel(fn, dim3(a.grid), dim3(a.block), args, a.dyn_smem, a.stream);
 }
 
-cudaError_t regroup_occupancy(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park, int* ctas)
+cudaError_t regroup_occupancy(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park, bool flat,
+                              int* ctas)
 {
-    const void* fn = regroup_fn(regs, profile, dyn_smem != 0u, park);
+    const void* fn = regroup_fn(regs, profile, dyn_smem != 0u, park, flat);
     if(!fn) return cudaErrorInvalidValue;
     if(dyn_smem)
     {

@@ -6,6 +6,7 @@
 // and the regrouping workspace (RAII on the host side of the ABI), copies
 // inputs in and outputs out, and runs the kernel to completion on the device
 // without per-round host round trips.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -18,6 +19,29 @@
 #include "runtime_iface.h"
 
 using namespace loom_b200;
+
+bool
+loom_b200::table_flat(const void* table, const unsigned long long words)
+{
+    if(!table) return true;
+    if(words) return words <= kFlatWords;
+    using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const Range range = []() -> Range
+    {
+        void*                           fn = nullptr;
+        cudaDriverEntryPointQueryResult q  = cudaDriverEntryPointSymbolNotFound;
+        if(cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+           q != cudaDriverEntryPointSuccess)
+            fn = nullptr;
+        cudaGetLastError();
+        return reinterpret_cast<Range>(fn);
+    }();
+    CUdeviceptr       base = 0;
+    size_t            size = 0;
+    const CUdeviceptr at   = reinterpret_cast<CUdeviceptr>(table);
+    if(!range || range(&base, &size, at) != CUDA_SUCCESS) return false;
+    return (base + size - at) / sizeof(uint32_t) <= kFlatWords;
+}
 
 namespace
 {
@@ -495,6 +519,7 @@ launch(loom_b200_handle* h, const loom_b200_launch& L, cudaStream_t stream, uint
     cols.inst_start = reinterpret_cast<const unsigned long long*>(L.instance_starts);
     cols.num_inst   = L.instance_starts ? L.num_instances : 0u;
     cols.table      = L.table;
+    cols.table_flat = table_flat(L.table, L.table_words) ? 1u : 0u;
     cols.tid_base   = first; // thread ids in flight lie in [first, first + n)
     const loom_b200_opts& o = h->opts;
     // a regrouping handle runs launches below plain_below threads on the
@@ -523,7 +548,8 @@ launch(loom_b200_handle* h, const loom_b200_launch& L, cudaStream_t stream, uint
             const unsigned    dyn = o.bulk_restore ? bulk_stage_bytes(block / 32u, e.max_stage_row) : 0u;
             const cudaError_t oe  = dyn > kMaxDynSmem ? cudaErrorInvalidValue
                                                       : e.regroup_occupancy(static_cast<int>(block), o.profile != 0,
-                                                                            o.max_regs, dyn, park_form(o), &ctas);
+                                                                            o.max_regs, dyn, park_form(o),
+                                                                            cols.table_flat != 0u, &ctas);
             if(oe == cudaErrorInvalidValue && dyn > kMaxDynSmem && block > 32)
             {
                 block /= 2; // the staging area of this many warps does not fit

@@ -66,13 +66,18 @@ struct KernelEntry
     cudaError_t (*plain)(const PlainLaunch&);
     cudaError_t (*regroup)(const RegroupLaunch&);
     cudaError_t (*regroup_occupancy)(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park,
-                                     int* ctas_per_sm);
+                                     bool flat, int* ctas_per_sm);
     const loom_b200_queue_layout* queues;   // num_queues entries
     const QueueSegment*           segments; // num_queues entries
     const unsigned*               reg_caps; // compiled register caps, default first
     unsigned                      num_reg_caps;
     unsigned                      max_stage_row; // K::kMaxStageRow (bulk_restore staging per entry)
 };
+
+/// Whether a launch's table is flat (Columns::table_flat): no table, or one
+/// of at most kFlatWords words.  Where the caller gives no word count, the
+/// device allocation that holds the table bounds it.
+bool table_flat(const void* table, unsigned long long words);
 
 extern const KernelEntry* const kRegistry[];
 extern const int                kRegistrySize;

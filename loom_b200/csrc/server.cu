@@ -265,6 +265,13 @@ dalloc(loom_b200_server* s, void** p, size_t bytes)
     return LOOM_B200_OK;
 }
 
+/// Whether the server's table (headers, then the arena) is flat.
+bool
+flat_table(const loom_b200_server_cfg& c)
+{
+    return c.max_requests * static_cast<uint64_t>(c.header_words) + c.table_words <= kFlatWords;
+}
+
 void
 free_all(loom_b200_server* s)
 {
@@ -450,7 +457,8 @@ loom_b200_server_create(const char*                 kernel,
     int      ctas  = 0;
     for(;;)
     {
-        if(e->regroup_occupancy(static_cast<int>(block), o.profile != 0, o.max_regs, 0u, true, &ctas) != cudaSuccess)
+        if(e->regroup_occupancy(static_cast<int>(block), o.profile != 0, o.max_regs, 0u, true,
+                                flat_table(*cfg), &ctas) != cudaSuccess)
         {
             delete s;
             return LOOM_B200_ERR_CUDA;
@@ -621,6 +629,7 @@ slice_launch(loom_b200_server* s, unsigned ctas_per_sm)
     c.inst_start = s->d_starts;
     c.num_inst   = static_cast<unsigned>(m);
     c.table      = s->d_table;
+    c.table_flat = flat_table(s->cfg) ? 1u : 0u;
     c.ring_mask  = s->mask;
     c.tid_base   = tid_base(s);
     c.inst_id    = s->d_ids;
@@ -658,7 +667,8 @@ slice_launch(loom_b200_server* s, unsigned ctas_per_sm)
         // never more CTAs per SM than fit (cooperative launches need every
         // CTA resident at once)
         int fit = 0;
-        SV_CUDA(s->e->regroup_occupancy(static_cast<int>(s->block), o.profile != 0, o.max_regs, 0u, true, &fit));
+        SV_CUDA(s->e->regroup_occupancy(static_cast<int>(s->block), o.profile != 0, o.max_regs, 0u, true,
+                                        flat_table(s->cfg), &fit));
         const unsigned c = std::min<unsigned>(ctas_per_sm, static_cast<unsigned>(std::max(fit, 1)));
         L.grid           = c * static_cast<unsigned>(s->sms);
     }

@@ -164,6 +164,7 @@ loom_b200_launch_static(const char*             kernel,
     cols.inst_start = reinterpret_cast<const unsigned long long*>(L->instance_starts);
     cols.num_inst   = L->instance_starts ? L->num_instances : 0u;
     cols.table      = L->table;
+    cols.table_flat = table_flat(L->table, L->table_words) ? 1u : 0u;
 
     loom_b200_opts o{};
     if(opts) o = *opts;
@@ -203,7 +204,7 @@ loom_b200_launch_static(const char*             kernel,
     int      ctas  = 0;
     for(;;)
     {
-        if(e->regroup_occupancy(static_cast<int>(block), false, 0u, 0u, true, &ctas) != cudaSuccess)
+        if(e->regroup_occupancy(static_cast<int>(block), false, 0u, 0u, true, cols.table_flat != 0u, &ctas) != cudaSuccess)
             return LOOM_B200_ERR_CUDA;
         if(ctas > 0 || block <= 32) break;
         block /= 2;
