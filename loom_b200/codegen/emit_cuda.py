@@ -615,8 +615,14 @@ def generate(k: Kernel) -> str:
     # back in reverse post-order): every cycle passes one, and the blocks in
     # between have no early exit, so a diverged warp reconverges at their
     # post-dominators as in straight CUDA
-    rank = k.rpo_ranks()
-    headers = {t for b in k.blocks for t in b.successors() if t != HALT and rank[t] <= rank[b.idx]}
+    headers = k.loop_headers()
+    # the regrouping engine's steps end at a minimal set of headers that
+    # every cycle passes: a step costs it some 30 instructions, and the path
+    # tracer's `bounce`, which runs into the intersection loop's own header,
+    # only added steps (1024x768x64 render 25.2 -> 24.6 ms without it); the
+    # long blocks stay, where lanes may have to wait for others.  The plain
+    # engine spends its step guard at every header.
+    steps = k.step_headers(set(long_blocks(k)))
     w("    // Runs the lane's own path from block `entry` for at most `budget`")
     w("    // loop iterations (visits of a loop header); returns the block it")
     w("    // stopped at, or kHalt.  With `stop_heavy`, a block whose quorum is")
@@ -624,8 +630,10 @@ def generate(k: Kernel) -> str:
     w("    // the warp's vote chose it.  A block that loops on itself takes up")
     w("    // to `spin` further iterations without spending budget (a loop the")
     w("    // warp's lanes run together needs no step of its own per iteration).")
-    w("    // kFlat: the launch's table is flat (Columns::table_flat).")
-    w("    template <bool kProf, bool kFlat>")
+    w("    // kFlat: the launch's table is flat (Columns::table_flat).  kAllHeaders:")
+    w("    // every loop header spends budget (the plain engine's step guard);")
+    w("    // otherwise a minimal set of them that every cycle passes.")
+    w("    template <bool kProf, bool kFlat, bool kAllHeaders>")
     w("    __device__ __forceinline__ static int")
     w("    run_burst(const int entry, Regs& R, Ctx& ctx, unsigned budget, const bool stop_heavy = false,")
     w("              unsigned spin = 0u)")
@@ -657,8 +665,12 @@ def generate(k: Kernel) -> str:
                 back = f"{{ if(spin != 0u) {{ --spin; goto L_B{blk.idx}_spin; }} goto L_B{blk.idx}_again; }}"
             transfer = [t.replace(own, back) for t in transfer]
         if blk.idx in headers:
-            w(f"        if(budget == 0u) return {blk.idx};")
-            w("        --budget;")
+            if blk.idx in steps:
+                w(f"        if(budget == 0u) return {blk.idx};")
+                w("        --budget;")
+            else:
+                w(f"        if(kAllHeaders && budget == 0u) return {blk.idx};")
+                w("        if(kAllHeaders) --budget;")
         if self_loop:
             w(f"    L_B{blk.idx}_spin:")
         if heavy:

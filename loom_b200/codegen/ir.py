@@ -383,6 +383,33 @@ class Kernel:
             rank[b] = r
         return rank
 
+    def loop_headers(self) -> Set[int]:
+        """Targets of the edges that go back in reverse post-order: every
+        cycle of the program passes one of them."""
+        rank = self.rpo_ranks()
+        return {t for b in self.blocks for t in b.successors() if t != HALT and rank[t] <= rank[b.idx]}
+
+    def _acyclic_without(self, cut: Set[int]) -> bool:
+        """Whether the CFG has no cycle that avoids the blocks in `cut`."""
+        left = {b.idx for b in self.blocks} - cut
+        while left:
+            leaf = next((b for b in left if not any(t in left for t in self.blocks[b].successors() if t != HALT)), None)
+            if leaf is None:
+                return False
+            left.discard(leaf)
+        return True
+
+    def step_headers(self, keep: Set[int] = frozenset()) -> Set[int]:
+        """A minimal subset of the loop headers that every cycle still
+        passes: headers that loop on themselves and those in `keep` stay, of
+        the others the shortest are left out first."""
+        heads = self.loop_headers()
+        counts = self.instr_counts()
+        for h in sorted(heads, key=lambda h: (counts[h], h)):
+            if h not in keep and h not in self.blocks[h].successors() and self._acyclic_without(heads - {h}):
+                heads = heads - {h}
+        return heads
+
     def state_regs(self) -> List[int]:
         """Registers that are live at the entry of some block: the columns of
         the regrouping engine's state file."""

@@ -42,7 +42,7 @@ plain_kernel(const Columns                  cols,
         const unsigned budget = max_steps < 0xffffffffull
                                     ? static_cast<unsigned>(max_steps)
                                     : 0xffffffffu;
-        if(K::template run_burst<kProf, kFlat>(0, R, ctx, budget) != kHalt)
+        if(K::template run_burst<kProf, kFlat, true>(0, R, ctx, budget) != kHalt)
             ctx.flag(kStatusStepLimit);
         K::store_outputs(R, cols, tid);
     }

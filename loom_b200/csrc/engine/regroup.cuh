@@ -465,16 +465,16 @@ regroup_kernel(const RegroupParams p)
                             // default (a few iterations let halted lanes take
                             // new threads while the others keep looping)
                             if(minpc && p.spin_iters && p.spin_iters <= 16u)
-                                pc = K::template run_burst<kProf, kFlat>(pc, R, ctx, 1u, false, 16u);
+                                pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, 1u, false, 16u);
                             else if(minpc && p.spin_iters && p.spin_iters <= 64u)
-                                pc = K::template run_burst<kProf, kFlat>(pc, R, ctx, 1u, false, 64u);
+                                pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, 1u, false, 64u);
                             else if(minpc)
-                                pc = K::template run_burst<kProf, kFlat>(pc, R, ctx, 1u, false, kSelfLoopSpin);
+                                pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, 1u, false, kSelfLoopSpin);
                             else
-                                pc = K::template run_burst<kProf, kFlat>(pc, R, ctx, p.burst, kPark && cost_on && p.schedule < 2u);
+                                pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, p.burst, kPark && cost_on && p.schedule < 2u);
                         }
                         else
-                            pc = K::template run_burst<kProf, kFlat>(pc, R, ctx, minpc ? 1u : p.burst,
+                            pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, minpc ? 1u : p.burst,
                                                               kPark && cost_on && p.schedule < 2u,
                                                               minpc ? (p.spin_iters ? p.spin_iters : kSelfLoopSpin) : 0u);
                     }

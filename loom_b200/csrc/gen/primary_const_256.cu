@@ -158,8 +158,10 @@ struct K
     // the warp's vote chose it.  A block that loops on itself takes up
     // to `spin` further iterations without spending budget (a loop the
     // warp's lanes run together needs no step of its own per iteration).
-    // kFlat: the launch's table is flat (Columns::table_flat).
-    template <bool kProf, bool kFlat>
+    // kFlat: the launch's table is flat (Columns::table_flat).  kAllHeaders:
+    // every loop header spends budget (the plain engine's step guard);
+    // otherwise a minimal set of them that every cycle passes.
+    template <bool kProf, bool kFlat, bool kAllHeaders>
     __device__ __forceinline__ static int
     run_burst(const int entry, Regs& R, Ctx& ctx, unsigned budget, const bool stop_heavy = false,
               unsigned spin = 0u)

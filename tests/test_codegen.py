@@ -130,3 +130,33 @@ def test_slot_packing_of_a_mixed_row():
     assert [(o, w, [i for i, _ in c]) for o, w, c in lay["slots"]] == [
         (0, 16, [0, 2]), (16, 16, [1, 3, 4, 5]), (32, 8, [6, "tid"]), (40, 1, [7])]
     assert lay["end"] == 48
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_step_headers_cut_every_cycle(name):
+    """The regrouping engine's step headers: loop headers, with every long
+    block and self-loop among them, such that no cycle avoids them and, of
+    the others, none could be left out."""
+    k = ir.load(name)
+    succ = k.succ_table()
+
+    def cycle_without(cut):
+        state = {}
+
+        def walk(b):
+            state[b] = 1
+            for t in succ[b]:
+                if t != HALT and t not in cut and (state.get(t) == 1 or (t not in state and walk(t))):
+                    return True
+            state[b] = 2
+            return False
+
+        return any(b not in cut and b not in state and walk(b) for b in range(k.num_blocks))
+
+    heads, steps, longs = k.loop_headers(), k.step_headers(set(E.long_blocks(k))), set(E.long_blocks(k))
+    assert steps <= heads and (longs & heads) <= steps
+    assert not cycle_without(heads) and not cycle_without(steps)
+    for h in steps - longs:
+        assert h in succ[h] or cycle_without(steps - {h})
+    if name == "sphere_pt_f32":
+        assert {k.blocks[h].label for h in steps} == {"isect", "roll"}
