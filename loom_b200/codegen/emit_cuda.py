@@ -158,6 +158,110 @@ def literal(op: Operand) -> str:
     return f"(({ct}){bits:#x}ull)"
 
 
+# Rough issue slots of operations that cost many (division and square root
+# with IEEE rounding, their slow paths left out); every other one counts 1.
+OP_COST = {"div": 10, "mod": 20, "sqrt": 9, "rsqrt": 18, "sin": 60, "cos": 60}
+
+# A region that only a condition needs moves behind it from this cost on (the
+# branch and the reconvergence after it take 3 to 4 instructions).  The path
+# tracer's intersection loop is issue-bound, a ray misses most spheres of a
+# random scene, and the root of its clamped discriminant, 0, takes the square
+# root's slow path (29 cycles a warp instead of 14): behind `hit = det >= 0`
+# 48 batched requests run 1.28x as fast (15.9 ms), the 1024x768x64 render 24.58
+# -> 23.69 ms, the serving burst 1.08x as fast.
+SINK_MIN_COST = 12
+
+
+def guarded_region(instrs, live_out, fixed):
+    """Work of a block that only matters while a condition register holds
+    true: (position of the instruction that sets the register, positions of
+    the work), or None.
+
+    Loom kernels are written without branches: `hit = det >= 0`, then the
+    root, the nearer of two distances, `hit = hit && t < tmin`, `tmin = hit ?
+    t : tmin`.  With the register false, `r = r && x` leaves it false, a
+    conditional move under it that keeps its own register does nothing, and
+    what else feeds only those has no effect, so a lane whose condition is
+    false may skip all of it.  The rest of the block (`fixed` positions are
+    part of it, as are instructions with side effects) runs after the region,
+    and only where that order gives the same values.  Of all conditions the
+    one with the costliest region is taken."""
+    best, best_cost = None, SINK_MIN_COST - 1
+    n = len(instrs)
+    last = n - 1 if n and not isinstance(instrs[-1], Compute) else n
+    for c in range(last):
+        h = instrs[c]
+        if h.op not in CMP and h.op not in LOGIC and h.op != "pacc":
+            continue
+        reg = h.dst.reg
+        known = {reg}  # registers that hold false while the condition does
+        noop = set()
+        for q in range(c + 1, last):
+            ins = instrs[q]
+            first = None if not ins.args or ins.args[0].is_literal else ins.args[0].reg
+            same = first == ins.dst.reg
+            if ins.op == "cmov" and first in known and ins.args[2] == ins.dst:
+                noop.add(q)
+            elif (
+                (ins.op == "pacc" and ins.optype[2] == "land" or ins.op == "land")
+                and first in known and same and ins.args[0] == ins.dst and ins.dst.type in INT_TYPES
+            ):
+                noop.add(q)
+            elif ins.dst.reg in known:
+                known.discard(ins.dst.reg)
+                if not known:
+                    break
+        # backwards: what is read while the condition is false
+        live = set(live_out) | ({r for r in instrs[-1].reads()} if last < n else set())
+        skip = set()
+        for q in range(last - 1, c, -1):
+            ins = instrs[q]
+            if q in noop and q not in fixed:
+                skip.add(q)
+            elif ins.dst.reg in live or q in fixed or ins.op == "assert_fp":
+                live.discard(ins.dst.reg)
+                live |= set(ins.reads())
+            else:
+                skip.add(q)
+        # the region in order, then the rest: cut where the order matters
+        inside = []
+        rest = []
+        for q in range(c + 1, last):
+            ins = instrs[q]
+            if q not in skip:
+                rest.append(q)
+                continue
+            if any(
+                instrs[r].dst.reg in ins.reads() or instrs[r].dst.reg == ins.dst.reg or ins.dst.reg in instrs[r].reads()
+                for r in rest
+            ):
+                # this one and all later ones stay where they are
+                rest.append(q)
+                continue
+            inside.append(q)
+        # what stays may not need, while the condition is false, a register
+        # that the region would have set: true by liveness for the skipped
+        # set as a whole, so a cut set is checked again
+        if len(inside) != len(skip):
+            live = set(live_out) | ({r for r in instrs[-1].reads()} if last < n else set())
+            ok = True
+            for q in range(last - 1, c, -1):
+                ins = instrs[q]
+                if q in inside:
+                    if q not in noop and ins.dst.reg in live:
+                        ok = False
+                        break
+                    continue
+                live.discard(ins.dst.reg)
+                live |= set(ins.reads())
+            if not ok:
+                continue
+        cost = sum(OP_COST.get(instrs[q].op, 1) for q in inside)
+        if cost > best_cost:
+            best, best_cost = (c, set(inside)), cost
+    return best
+
+
 class Lowering:
     def __init__(self, k: Kernel):
         self.k = k
@@ -307,15 +411,17 @@ class Lowering:
                 member[p] = (first, d)
         return rows, member
 
-    def body(self, instrs, indent: str) -> List[str]:
+    def body(self, instrs, indent: str, live_out=None) -> List[str]:
+        """The instructions of a block (without its terminator).  `live_out`:
+        registers read after them, which allows work that only a condition
+        needs to move behind it."""
         rows, member = self.table_rows(instrs)
-        out = []
-        for pos, ins in enumerate(instrs):
-            if not isinstance(ins, Compute):
-                continue
+
+        def emit(pos: int, indent: str) -> List[str]:
+            out = []
+            ins = instrs[pos]
             if pos in rows:
                 base, dist = rows[pos]
-                out.append(indent + f"unsigned {', '.join(f'tw{pos}_{d}' for d in dist)};")
                 out.append(indent + f"const unsigned tb{pos} = static_cast<unsigned>({base});")
                 out.append(indent + "if constexpr(kFlat)")
                 out.append(indent + "{")
@@ -332,8 +438,30 @@ class Lowering:
                 out.append(indent + self.write(ins.dst, f"bitcast<{CTYPE[t]}>(tw{first}_{d})"))
             else:
                 out.append(indent + self.write(ins.dst, self.expr(ins)))
+            return out
+
+        todo = [p for p, ins in enumerate(instrs) if isinstance(ins, Compute)]
+        out = []
+        inner = indent + "    " if rows else indent
+        for pos in rows:
+            out.append(inner + f"unsigned {', '.join(f'tw{pos}_{d}' for d in rows[pos][1])};")
+        sink = guarded_region(instrs, live_out, set(rows) | set(member)) if live_out is not None else None
+        if sink:
+            cond, inside = sink
+            for p in todo:
+                if p <= cond:
+                    out.extend(emit(p, inner))
+            out.append(inner + f"if({self.read(instrs[cond].dst)})")
+            out.append(inner + "{")
+            for p in todo:
+                if p in inside:
+                    out.extend(emit(p, inner + "    "))
+            out.append(inner + "}")
+            todo = [p for p in todo if p > cond and p not in inside]
+        for p in todo:
+            out.extend(emit(p, inner))
         if rows:  # a scope of their own: labels of other blocks are jumped to past them
-            out = [indent + "{"] + ["    " + ln for ln in out] + [indent + "}"]
+            out = [indent + "{"] + out + [indent + "}"]
         return out
 
     # ------------------------------------------------------------ transfers
@@ -429,7 +557,7 @@ def generate(k: Kernel) -> str:
     nb = k.num_blocks
     nin = len(k.inputs)
     nout = len(k.outputs)
-    live_in, _ = k.liveness()
+    live_in, live_outs = k.liveness()
     state = k.state_regs()
     counts = k.instr_counts()
     live_bytes = [sum(L.regs[r].nbytes for r in li) for li in live_in]
@@ -676,7 +804,7 @@ def generate(k: Kernel) -> str:
         if heavy:
             w("        fresh = false;")
         w(f"        if constexpr(kProf) count_block(ctx, {blk.idx}, {len(blk.instrs)}u);")
-        o.extend(L.body(blk.instrs, "        "))
+        o.extend(L.body(blk.instrs, "        ", live_outs[blk.idx]))
         o.extend(transfer)
     w("    L_HALT:")
     w("        return kHalt;")

@@ -1197,23 +1197,26 @@ struct K
         fresh = false;
         if constexpr(kProf) count_block(ctx, 38, 19u);
         R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0xaull))));
-        R.r45 = static_cast<float>(static_cast<float>(static_cast<float>(R.r22) - static_cast<float>((0x1.0000000000000p-1f))));
-        R.r46 = static_cast<float>(static_cast<float>(static_cast<float>(R.r23) - static_cast<float>((-0x1.6666660000000p-2f))));
-        R.r47 = static_cast<float>(static_cast<float>(static_cast<float>(R.r24) - static_cast<float>((-0x1.3333340000000p-2f))));
-        R.r8 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
-        R.r8 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r45, R.r45, bitcast<float>(R.r8))));
-        R.r8 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r46, R.r46, bitcast<float>(R.r8))));
-        R.r8 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r47, R.r47, bitcast<float>(R.r8))));
-        R.r8 = bitcast<unsigned int>(static_cast<float>(op_rsqrt(static_cast<float>(bitcast<float>(R.r8)))));
-        R.r45 = static_cast<float>(static_cast<float>(static_cast<float>(R.r45) * static_cast<float>(bitcast<float>(R.r8))));
-        R.r46 = static_cast<float>(static_cast<float>(static_cast<float>(R.r46) * static_cast<float>(bitcast<float>(R.r8))));
-        R.r47 = static_cast<float>(static_cast<float>(static_cast<float>(R.r47) * static_cast<float>(bitcast<float>(R.r8))));
+        if(R.r14)
+        {
+            R.r45 = static_cast<float>(static_cast<float>(static_cast<float>(R.r22) - static_cast<float>((0x1.0000000000000p-1f))));
+            R.r46 = static_cast<float>(static_cast<float>(static_cast<float>(R.r23) - static_cast<float>((-0x1.6666660000000p-2f))));
+            R.r47 = static_cast<float>(static_cast<float>(static_cast<float>(R.r24) - static_cast<float>((-0x1.3333340000000p-2f))));
+            R.r8 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
+            R.r8 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r45, R.r45, bitcast<float>(R.r8))));
+            R.r8 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r46, R.r46, bitcast<float>(R.r8))));
+            R.r8 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r47, R.r47, bitcast<float>(R.r8))));
+            R.r8 = bitcast<unsigned int>(static_cast<float>(op_rsqrt(static_cast<float>(bitcast<float>(R.r8)))));
+            R.r45 = static_cast<float>(static_cast<float>(static_cast<float>(R.r45) * static_cast<float>(bitcast<float>(R.r8))));
+            R.r46 = static_cast<float>(static_cast<float>(static_cast<float>(R.r46) * static_cast<float>(bitcast<float>(R.r8))));
+            R.r47 = static_cast<float>(static_cast<float>(static_cast<float>(R.r47) * static_cast<float>(bitcast<float>(R.r8))));
+            R.r62 = static_cast<float>(((R.r14) ? (R.r45) : (R.r62)));
+            R.r63 = static_cast<float>(((R.r14) ? (R.r46) : (R.r63)));
+            R.r64 = static_cast<float>(((R.r14) ? (R.r47) : (R.r64)));
+        }
         R.r65 = static_cast<float>((0x0.0p+0f));
         R.r66 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : ((-0x1.0000000000000p+0f))));
         R.r67 = static_cast<float>((0x0.0p+0f));
-        R.r62 = static_cast<float>(((R.r14) ? (R.r45) : (R.r62)));
-        R.r63 = static_cast<float>(((R.r14) ? (R.r46) : (R.r63)));
-        R.r64 = static_cast<float>(((R.r14) ? (R.r47) : (R.r64)));
         goto L_B41;
     L_B39: // compute_sphere_normal
         fresh = false;

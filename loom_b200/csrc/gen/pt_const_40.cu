@@ -1141,23 +1141,26 @@ struct K
         fresh = false;
         if constexpr(kProf) count_block(ctx, 37, 19u);
         R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0xaull))));
-        R.r42 = static_cast<float>(static_cast<float>(static_cast<float>(R.r22) - static_cast<float>((0x1.0000000000000p-1f))));
-        R.r43 = static_cast<float>(static_cast<float>(static_cast<float>(R.r23) - static_cast<float>((-0x1.6666660000000p-2f))));
-        R.r44 = static_cast<float>(static_cast<float>(static_cast<float>(R.r24) - static_cast<float>((-0x1.3333340000000p-2f))));
-        R.r10 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
-        R.r10 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r42, R.r42, bitcast<float>(R.r10))));
-        R.r10 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r43, R.r43, bitcast<float>(R.r10))));
-        R.r10 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r44, R.r44, bitcast<float>(R.r10))));
-        R.r10 = bitcast<unsigned int>(static_cast<float>(op_rsqrt(static_cast<float>(bitcast<float>(R.r10)))));
-        R.r42 = static_cast<float>(static_cast<float>(static_cast<float>(R.r42) * static_cast<float>(bitcast<float>(R.r10))));
-        R.r43 = static_cast<float>(static_cast<float>(static_cast<float>(R.r43) * static_cast<float>(bitcast<float>(R.r10))));
-        R.r44 = static_cast<float>(static_cast<float>(static_cast<float>(R.r44) * static_cast<float>(bitcast<float>(R.r10))));
+        if(R.r14)
+        {
+            R.r42 = static_cast<float>(static_cast<float>(static_cast<float>(R.r22) - static_cast<float>((0x1.0000000000000p-1f))));
+            R.r43 = static_cast<float>(static_cast<float>(static_cast<float>(R.r23) - static_cast<float>((-0x1.6666660000000p-2f))));
+            R.r44 = static_cast<float>(static_cast<float>(static_cast<float>(R.r24) - static_cast<float>((-0x1.3333340000000p-2f))));
+            R.r10 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
+            R.r10 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r42, R.r42, bitcast<float>(R.r10))));
+            R.r10 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r43, R.r43, bitcast<float>(R.r10))));
+            R.r10 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r44, R.r44, bitcast<float>(R.r10))));
+            R.r10 = bitcast<unsigned int>(static_cast<float>(op_rsqrt(static_cast<float>(bitcast<float>(R.r10)))));
+            R.r42 = static_cast<float>(static_cast<float>(static_cast<float>(R.r42) * static_cast<float>(bitcast<float>(R.r10))));
+            R.r43 = static_cast<float>(static_cast<float>(static_cast<float>(R.r43) * static_cast<float>(bitcast<float>(R.r10))));
+            R.r44 = static_cast<float>(static_cast<float>(static_cast<float>(R.r44) * static_cast<float>(bitcast<float>(R.r10))));
+            R.r59 = static_cast<float>(((R.r14) ? (R.r42) : (R.r59)));
+            R.r60 = static_cast<float>(((R.r14) ? (R.r43) : (R.r60)));
+            R.r61 = static_cast<float>(((R.r14) ? (R.r44) : (R.r61)));
+        }
         R.r62 = static_cast<float>((0x0.0p+0f));
         R.r63 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : ((-0x1.0000000000000p+0f))));
         R.r64 = static_cast<float>((0x0.0p+0f));
-        R.r59 = static_cast<float>(((R.r14) ? (R.r42) : (R.r59)));
-        R.r60 = static_cast<float>(((R.r14) ? (R.r43) : (R.r60)));
-        R.r61 = static_cast<float>(((R.r14) ? (R.r44) : (R.r61)));
         goto L_B40;
     L_B38: // compute_sphere_normal
         fresh = false;

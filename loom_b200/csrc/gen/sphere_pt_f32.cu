@@ -308,8 +308,8 @@ struct K
         fresh = false;
         if constexpr(kProf) count_block(ctx, 0, 32u);
         {
-            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) * static_cast<unsigned int>(((unsigned int)0x10ull))));
             unsigned tw1_0, tw1_1, tw1_2, tw1_3, tw1_4, tw1_5, tw1_6, tw1_7, tw1_8, tw1_9;
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) * static_cast<unsigned int>(((unsigned int)0x10ull))));
             const unsigned tb1 = static_cast<unsigned>(R.r6);
             if constexpr(kFlat)
             {
@@ -498,16 +498,19 @@ struct K
             R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
             R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
             R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
-            R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
-            R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
-            R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
-            R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
-            R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
-            R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
-            R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
-            R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
-            R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
-            R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+            if(R.r71)
+            {
+                R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
+                R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
+                R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
+                R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
+                R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
+                R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
+                R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
+                R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
+                R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
+                R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+            }
             R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
             R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
             R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
@@ -524,9 +527,9 @@ struct K
         fresh = false;
         if constexpr(kProf) count_block(ctx, 5, 28u);
         {
+            unsigned tw2_0, tw2_1, tw2_2, tw2_3, tw2_4, tw2_5, tw2_6, tw2_7;
             R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r54) * static_cast<unsigned int>(((unsigned int)0x8ull))));
             R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(R.r12)));
-            unsigned tw2_0, tw2_1, tw2_2, tw2_3, tw2_4, tw2_5, tw2_6, tw2_7;
             const unsigned tb2 = static_cast<unsigned>(R.r56);
             if constexpr(kFlat)
             {
