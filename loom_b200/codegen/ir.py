@@ -383,6 +383,17 @@ class Kernel:
             rank[b] = r
         return rank
 
+    def reachable(self, b: int) -> Set[int]:
+        """Blocks on the paths from block `b` (itself included; none: HALT)."""
+        seen: Set[int] = set()
+        todo = [b]
+        while todo:
+            x = todo.pop()
+            if x != HALT and x not in seen:
+                seen.add(x)
+                todo.extend(self.blocks[x].successors())
+        return seen
+
     def loop_headers(self) -> Set[int]:
         """Targets of the edges that go back in reverse post-order: every
         cycle of the program passes one of them."""

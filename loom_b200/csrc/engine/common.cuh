@@ -7,6 +7,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 
 #include "loom_b200.h"
 
@@ -112,6 +113,37 @@ __device__ __forceinline__ T
 op_min(const T a, const T b)
 {
     return (b < a) ? b : a;
+}
+
+// Iterations of a loop `do { ...; ++i; } while(i cmp n)` after which it
+// surely goes on, at most `most`: the k for which i + k cmp n holds from k = 1
+// on (they do not wrap, but for !=, whose distance wraps as the counter does).
+template <typename T>
+__device__ __forceinline__ unsigned
+loop_more(const T d, const unsigned most)
+{
+    return d < static_cast<T>(most) ? static_cast<unsigned>(d) : most;
+}
+template <typename T>
+__device__ __forceinline__ unsigned
+loop_more_lt(const T i, const T n, const unsigned most)
+{
+    using U = std::make_unsigned_t<T>;
+    return i < n ? loop_more<U>(static_cast<U>(n) - static_cast<U>(i) - 1u, most) : 0u;
+}
+template <typename T>
+__device__ __forceinline__ unsigned
+loop_more_le(const T i, const T n, const unsigned most)
+{
+    using U = std::make_unsigned_t<T>;
+    return i < n ? loop_more<U>(static_cast<U>(n) - static_cast<U>(i), most) : 0u;
+}
+template <typename T>
+__device__ __forceinline__ unsigned
+loop_more_ne(const T i, const T n, const unsigned most)
+{
+    using U = std::make_unsigned_t<T>;
+    return loop_more<U>(static_cast<U>(n) - static_cast<U>(i) - 1u, most);
 }
 
 __device__ __forceinline__ float op_abs(float v) { return fabsf(v); }

@@ -114,6 +114,9 @@ struct K
         (void)ctx;
         (void)stop_heavy;
         (void)spin;
+        unsigned left = 0u; // iterations of a self-loop left
+        unsigned sure = 0u; // of them, those that surely go on
+        (void)sure;
         bool fresh = true; // no block run yet in this burst
         (void)fresh;
         switch(entry)
@@ -134,18 +137,107 @@ struct K
         if(stop_heavy && !fresh) return 1;
     L_B1_again:
         if(budget == 0u) return 1;
-        --budget;
-    L_B1_spin:
-        fresh = false;
-        if constexpr(kProf) count_block(ctx, 1, 8u);
-        R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-        R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-        R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
-        R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-        R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
-        R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-        R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-        if(R.r3) { if(spin != 0u) { --spin; goto L_B1_spin; } goto L_B1_again; } else goto L_HALT;
+        left = spin ? spin : budget;
+        while(left >= 8u)
+        {
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 1, 8u);
+            R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            if(!(R.r3)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 1, 8u);
+            R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            if(!(R.r3)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 1, 8u);
+            R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            if(!(R.r3)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 1, 8u);
+            R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            if(!(R.r3)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 1, 8u);
+            R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            if(!(R.r3)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 1, 8u);
+            R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            if(!(R.r3)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 1, 8u);
+            R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            if(!(R.r3)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 1, 8u);
+            R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            if(!(R.r3)) goto L_HALT;
+            left -= 8u;
+        }
+        while(left)
+        {
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 1, 8u);
+            R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
+            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            --left;
+            if(!(R.r3)) goto L_HALT;
+        }
+        if(spin) { spin = 0u; --budget; } else budget = 0u;
+        goto L_B1_again;
     L_HALT:
         return kHalt;
     }

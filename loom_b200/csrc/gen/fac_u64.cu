@@ -111,6 +111,9 @@ struct K
         (void)ctx;
         (void)stop_heavy;
         (void)spin;
+        unsigned left = 0u; // iterations of a self-loop left
+        unsigned sure = 0u; // of them, those that surely go on
+        (void)sure;
         bool fresh = true; // no block run yet in this burst
         (void)fresh;
         switch(entry)
@@ -137,14 +140,71 @@ struct K
         if(stop_heavy && !fresh) return 2;
     L_B2_again:
         if(budget == 0u) return 2;
-        --budget;
-    L_B2_spin:
-        fresh = false;
-        if constexpr(kProf) count_block(ctx, 2, 4u);
-        R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
-        R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-        R.r2 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r3) == static_cast<unsigned long long>(((unsigned long long)0x0ull))));
-        if(R.r2) goto L_HALT; else { if(spin != 0u) { --spin; goto L_B2_spin; } goto L_B2_again; }
+        left = spin ? spin : budget;
+        while(left >= 8u)
+        {
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 4u);
+            R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
+            R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r2 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r3) == static_cast<unsigned long long>(((unsigned long long)0x0ull))));
+            if(!!(R.r2)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 4u);
+            R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
+            R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r2 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r3) == static_cast<unsigned long long>(((unsigned long long)0x0ull))));
+            if(!!(R.r2)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 4u);
+            R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
+            R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r2 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r3) == static_cast<unsigned long long>(((unsigned long long)0x0ull))));
+            if(!!(R.r2)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 4u);
+            R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
+            R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r2 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r3) == static_cast<unsigned long long>(((unsigned long long)0x0ull))));
+            if(!!(R.r2)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 4u);
+            R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
+            R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r2 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r3) == static_cast<unsigned long long>(((unsigned long long)0x0ull))));
+            if(!!(R.r2)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 4u);
+            R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
+            R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r2 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r3) == static_cast<unsigned long long>(((unsigned long long)0x0ull))));
+            if(!!(R.r2)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 4u);
+            R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
+            R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r2 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r3) == static_cast<unsigned long long>(((unsigned long long)0x0ull))));
+            if(!!(R.r2)) goto L_HALT;
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 4u);
+            R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
+            R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r2 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r3) == static_cast<unsigned long long>(((unsigned long long)0x0ull))));
+            if(!!(R.r2)) goto L_HALT;
+            left -= 8u;
+        }
+        while(left)
+        {
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 4u);
+            R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
+            R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r2 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r3) == static_cast<unsigned long long>(((unsigned long long)0x0ull))));
+            --left;
+            if(!!(R.r2)) goto L_HALT;
+        }
+        if(spin) { spin = 0u; --budget; } else budget = 0u;
+        goto L_B2_again;
     L_HALT:
         return kHalt;
     }

@@ -114,6 +114,9 @@ struct K
         (void)ctx;
         (void)stop_heavy;
         (void)spin;
+        unsigned left = 0u; // iterations of a self-loop left
+        unsigned sure = 0u; // of them, those that surely go on
+        (void)sure;
         bool fresh = true; // no block run yet in this burst
         (void)fresh;
         switch(entry)
@@ -144,16 +147,134 @@ struct K
         if(stop_heavy && !fresh) return 2;
     L_B2_again:
         if(budget == 0u) return 2;
-        --budget;
-    L_B2_spin:
-        fresh = false;
-        if constexpr(kProf) count_block(ctx, 2, 6u);
-        R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
-        R.r4 = static_cast<unsigned int>(R.r2);
-        R.r2 = static_cast<unsigned int>(R.r6);
-        R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-        R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
-        if(R.r3) { if(spin != 0u) { --spin; goto L_B2_spin; } goto L_B2_again; } else goto L_HALT;
+        left = spin ? spin : budget;
+        sure = loop_more_le<unsigned int>(R.r5, R.r1, left);
+        left -= sure;
+        while(sure >= 8u)
+        {
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            sure -= 8u;
+        }
+        if(sure >= 4u)
+        {
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            sure -= 4u;
+        }
+        if(sure >= 2u)
+        {
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            sure -= 2u;
+        }
+        left += sure;
+        while(left)
+        {
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 2, 6u);
+            R.r6 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r4) + static_cast<unsigned int>(R.r2)));
+            R.r4 = static_cast<unsigned int>(R.r2);
+            R.r2 = static_cast<unsigned int>(R.r6);
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r3 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r5) <= static_cast<unsigned int>(R.r1)));
+            --left;
+            if(!(R.r3)) goto L_HALT;
+        }
+        if(spin) { spin = 0u; --budget; } else budget = 0u;
+        goto L_B2_again;
     L_HALT:
         return kHalt;
     }

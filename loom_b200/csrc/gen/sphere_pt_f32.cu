@@ -272,6 +272,9 @@ struct K
         (void)ctx;
         (void)stop_heavy;
         (void)spin;
+        unsigned left = 0u; // iterations of a self-loop left
+        unsigned sure = 0u; // of them, those that surely go on
+        (void)sure;
         bool fresh = true; // no block run yet in this burst
         (void)fresh;
         switch(entry)
@@ -452,70 +455,455 @@ struct K
         if(stop_heavy && !fresh) return 3;
     L_B3_again:
         if(budget == 0u) return 3;
-        --budget;
-    L_B3_spin:
-        fresh = false;
-        if constexpr(kProf) count_block(ctx, 3, 38u);
+        left = spin ? spin : budget;
+        sure = loop_more_lt<unsigned int>(R.r55, R.r13, left);
+        left -= sure;
+        while(sure >= 4u)
         {
-            unsigned tw0_0, tw0_1, tw0_2, tw0_3;
-            const unsigned tb0 = static_cast<unsigned>(R.r56);
-            if constexpr(kFlat)
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 3, 38u);
             {
-                const unsigned* tp = ctx.cols->table + tb0;
-                tw0_0 = __ldg(tp + 0);
-                tw0_1 = __ldg(tp + 1);
-                tw0_2 = __ldg(tp + 2);
-                tw0_3 = __ldg(tp + 3);
+                unsigned tw0_0, tw0_1, tw0_2, tw0_3;
+                const unsigned tb0 = static_cast<unsigned>(R.r56);
+                if constexpr(kFlat)
+                {
+                    const unsigned* tp = ctx.cols->table + tb0;
+                    tw0_0 = __ldg(tp + 0);
+                    tw0_1 = __ldg(tp + 1);
+                    tw0_2 = __ldg(tp + 2);
+                    tw0_3 = __ldg(tp + 3);
+                }
+                else
+                {
+                    tw0_0 = table_load<unsigned>(*ctx.cols, tb0 + 0u);
+                    tw0_1 = table_load<unsigned>(*ctx.cols, tb0 + 1u);
+                    tw0_2 = table_load<unsigned>(*ctx.cols, tb0 + 2u);
+                    tw0_3 = table_load<unsigned>(*ctx.cols, tb0 + 3u);
+                }
+                R.r57 = static_cast<float>(bitcast<float>(tw0_0));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r58 = static_cast<float>(bitcast<float>(tw0_1));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
+                R.r59 = static_cast<float>(bitcast<float>(tw0_2));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
+                R.r60 = static_cast<float>(bitcast<float>(tw0_3));
+                R.r61 = static_cast<float>(static_cast<float>(static_cast<float>(R.r57) - static_cast<float>(R.r46)));
+                R.r62 = static_cast<float>(static_cast<float>(static_cast<float>(R.r58) - static_cast<float>(R.r47)));
+                R.r63 = static_cast<float>(static_cast<float>(static_cast<float>(R.r59) - static_cast<float>(R.r48)));
+                R.r64 = static_cast<float>((0x0.0p+0f));
+                R.r64 = static_cast<float>(op_fma(R.r61, R.r42, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r62, R.r43, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r63, R.r44, R.r64));
+                R.r65 = static_cast<float>(static_cast<float>(-static_cast<float>(R.r64)));
+                R.r66 = static_cast<float>(op_fma(R.r65, R.r42, R.r61));
+                R.r67 = static_cast<float>(op_fma(R.r65, R.r43, R.r62));
+                R.r68 = static_cast<float>(op_fma(R.r65, R.r44, R.r63));
+                R.r69 = static_cast<float>((0x0.0p+0f));
+                R.r69 = static_cast<float>(op_fma(R.r66, R.r66, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r67, R.r67, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
+                R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
+                R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
+                if(R.r71)
+                {
+                    R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
+                    R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
+                    R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
+                    R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
+                    R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
+                    R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
+                    R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
+                    R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+                }
+                R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
+                R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
             }
-            else
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 3, 38u);
             {
-                tw0_0 = table_load<unsigned>(*ctx.cols, tb0 + 0u);
-                tw0_1 = table_load<unsigned>(*ctx.cols, tb0 + 1u);
-                tw0_2 = table_load<unsigned>(*ctx.cols, tb0 + 2u);
-                tw0_3 = table_load<unsigned>(*ctx.cols, tb0 + 3u);
+                unsigned tw0_0, tw0_1, tw0_2, tw0_3;
+                const unsigned tb0 = static_cast<unsigned>(R.r56);
+                if constexpr(kFlat)
+                {
+                    const unsigned* tp = ctx.cols->table + tb0;
+                    tw0_0 = __ldg(tp + 0);
+                    tw0_1 = __ldg(tp + 1);
+                    tw0_2 = __ldg(tp + 2);
+                    tw0_3 = __ldg(tp + 3);
+                }
+                else
+                {
+                    tw0_0 = table_load<unsigned>(*ctx.cols, tb0 + 0u);
+                    tw0_1 = table_load<unsigned>(*ctx.cols, tb0 + 1u);
+                    tw0_2 = table_load<unsigned>(*ctx.cols, tb0 + 2u);
+                    tw0_3 = table_load<unsigned>(*ctx.cols, tb0 + 3u);
+                }
+                R.r57 = static_cast<float>(bitcast<float>(tw0_0));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r58 = static_cast<float>(bitcast<float>(tw0_1));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
+                R.r59 = static_cast<float>(bitcast<float>(tw0_2));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
+                R.r60 = static_cast<float>(bitcast<float>(tw0_3));
+                R.r61 = static_cast<float>(static_cast<float>(static_cast<float>(R.r57) - static_cast<float>(R.r46)));
+                R.r62 = static_cast<float>(static_cast<float>(static_cast<float>(R.r58) - static_cast<float>(R.r47)));
+                R.r63 = static_cast<float>(static_cast<float>(static_cast<float>(R.r59) - static_cast<float>(R.r48)));
+                R.r64 = static_cast<float>((0x0.0p+0f));
+                R.r64 = static_cast<float>(op_fma(R.r61, R.r42, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r62, R.r43, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r63, R.r44, R.r64));
+                R.r65 = static_cast<float>(static_cast<float>(-static_cast<float>(R.r64)));
+                R.r66 = static_cast<float>(op_fma(R.r65, R.r42, R.r61));
+                R.r67 = static_cast<float>(op_fma(R.r65, R.r43, R.r62));
+                R.r68 = static_cast<float>(op_fma(R.r65, R.r44, R.r63));
+                R.r69 = static_cast<float>((0x0.0p+0f));
+                R.r69 = static_cast<float>(op_fma(R.r66, R.r66, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r67, R.r67, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
+                R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
+                R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
+                if(R.r71)
+                {
+                    R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
+                    R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
+                    R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
+                    R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
+                    R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
+                    R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
+                    R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
+                    R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+                }
+                R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
+                R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
             }
-            R.r57 = static_cast<float>(bitcast<float>(tw0_0));
-            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r58 = static_cast<float>(bitcast<float>(tw0_1));
-            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
-            R.r59 = static_cast<float>(bitcast<float>(tw0_2));
-            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
-            R.r60 = static_cast<float>(bitcast<float>(tw0_3));
-            R.r61 = static_cast<float>(static_cast<float>(static_cast<float>(R.r57) - static_cast<float>(R.r46)));
-            R.r62 = static_cast<float>(static_cast<float>(static_cast<float>(R.r58) - static_cast<float>(R.r47)));
-            R.r63 = static_cast<float>(static_cast<float>(static_cast<float>(R.r59) - static_cast<float>(R.r48)));
-            R.r64 = static_cast<float>((0x0.0p+0f));
-            R.r64 = static_cast<float>(op_fma(R.r61, R.r42, R.r64));
-            R.r64 = static_cast<float>(op_fma(R.r62, R.r43, R.r64));
-            R.r64 = static_cast<float>(op_fma(R.r63, R.r44, R.r64));
-            R.r65 = static_cast<float>(static_cast<float>(-static_cast<float>(R.r64)));
-            R.r66 = static_cast<float>(op_fma(R.r65, R.r42, R.r61));
-            R.r67 = static_cast<float>(op_fma(R.r65, R.r43, R.r62));
-            R.r68 = static_cast<float>(op_fma(R.r65, R.r44, R.r63));
-            R.r69 = static_cast<float>((0x0.0p+0f));
-            R.r69 = static_cast<float>(op_fma(R.r66, R.r66, R.r69));
-            R.r69 = static_cast<float>(op_fma(R.r67, R.r67, R.r69));
-            R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
-            R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
-            R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
-            if(R.r71)
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 3, 38u);
             {
-                R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
-                R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
-                R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
-                R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
-                R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
-                R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
-                R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
-                R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
-                R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
-                R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+                unsigned tw0_0, tw0_1, tw0_2, tw0_3;
+                const unsigned tb0 = static_cast<unsigned>(R.r56);
+                if constexpr(kFlat)
+                {
+                    const unsigned* tp = ctx.cols->table + tb0;
+                    tw0_0 = __ldg(tp + 0);
+                    tw0_1 = __ldg(tp + 1);
+                    tw0_2 = __ldg(tp + 2);
+                    tw0_3 = __ldg(tp + 3);
+                }
+                else
+                {
+                    tw0_0 = table_load<unsigned>(*ctx.cols, tb0 + 0u);
+                    tw0_1 = table_load<unsigned>(*ctx.cols, tb0 + 1u);
+                    tw0_2 = table_load<unsigned>(*ctx.cols, tb0 + 2u);
+                    tw0_3 = table_load<unsigned>(*ctx.cols, tb0 + 3u);
+                }
+                R.r57 = static_cast<float>(bitcast<float>(tw0_0));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r58 = static_cast<float>(bitcast<float>(tw0_1));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
+                R.r59 = static_cast<float>(bitcast<float>(tw0_2));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
+                R.r60 = static_cast<float>(bitcast<float>(tw0_3));
+                R.r61 = static_cast<float>(static_cast<float>(static_cast<float>(R.r57) - static_cast<float>(R.r46)));
+                R.r62 = static_cast<float>(static_cast<float>(static_cast<float>(R.r58) - static_cast<float>(R.r47)));
+                R.r63 = static_cast<float>(static_cast<float>(static_cast<float>(R.r59) - static_cast<float>(R.r48)));
+                R.r64 = static_cast<float>((0x0.0p+0f));
+                R.r64 = static_cast<float>(op_fma(R.r61, R.r42, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r62, R.r43, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r63, R.r44, R.r64));
+                R.r65 = static_cast<float>(static_cast<float>(-static_cast<float>(R.r64)));
+                R.r66 = static_cast<float>(op_fma(R.r65, R.r42, R.r61));
+                R.r67 = static_cast<float>(op_fma(R.r65, R.r43, R.r62));
+                R.r68 = static_cast<float>(op_fma(R.r65, R.r44, R.r63));
+                R.r69 = static_cast<float>((0x0.0p+0f));
+                R.r69 = static_cast<float>(op_fma(R.r66, R.r66, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r67, R.r67, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
+                R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
+                R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
+                if(R.r71)
+                {
+                    R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
+                    R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
+                    R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
+                    R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
+                    R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
+                    R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
+                    R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
+                    R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+                }
+                R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
+                R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
             }
-            R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
-            R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 3, 38u);
+            {
+                unsigned tw0_0, tw0_1, tw0_2, tw0_3;
+                const unsigned tb0 = static_cast<unsigned>(R.r56);
+                if constexpr(kFlat)
+                {
+                    const unsigned* tp = ctx.cols->table + tb0;
+                    tw0_0 = __ldg(tp + 0);
+                    tw0_1 = __ldg(tp + 1);
+                    tw0_2 = __ldg(tp + 2);
+                    tw0_3 = __ldg(tp + 3);
+                }
+                else
+                {
+                    tw0_0 = table_load<unsigned>(*ctx.cols, tb0 + 0u);
+                    tw0_1 = table_load<unsigned>(*ctx.cols, tb0 + 1u);
+                    tw0_2 = table_load<unsigned>(*ctx.cols, tb0 + 2u);
+                    tw0_3 = table_load<unsigned>(*ctx.cols, tb0 + 3u);
+                }
+                R.r57 = static_cast<float>(bitcast<float>(tw0_0));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r58 = static_cast<float>(bitcast<float>(tw0_1));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
+                R.r59 = static_cast<float>(bitcast<float>(tw0_2));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
+                R.r60 = static_cast<float>(bitcast<float>(tw0_3));
+                R.r61 = static_cast<float>(static_cast<float>(static_cast<float>(R.r57) - static_cast<float>(R.r46)));
+                R.r62 = static_cast<float>(static_cast<float>(static_cast<float>(R.r58) - static_cast<float>(R.r47)));
+                R.r63 = static_cast<float>(static_cast<float>(static_cast<float>(R.r59) - static_cast<float>(R.r48)));
+                R.r64 = static_cast<float>((0x0.0p+0f));
+                R.r64 = static_cast<float>(op_fma(R.r61, R.r42, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r62, R.r43, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r63, R.r44, R.r64));
+                R.r65 = static_cast<float>(static_cast<float>(-static_cast<float>(R.r64)));
+                R.r66 = static_cast<float>(op_fma(R.r65, R.r42, R.r61));
+                R.r67 = static_cast<float>(op_fma(R.r65, R.r43, R.r62));
+                R.r68 = static_cast<float>(op_fma(R.r65, R.r44, R.r63));
+                R.r69 = static_cast<float>((0x0.0p+0f));
+                R.r69 = static_cast<float>(op_fma(R.r66, R.r66, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r67, R.r67, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
+                R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
+                R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
+                if(R.r71)
+                {
+                    R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
+                    R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
+                    R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
+                    R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
+                    R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
+                    R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
+                    R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
+                    R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+                }
+                R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
+                R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
+            }
+            sure -= 4u;
         }
-        if(R.r33) { if(spin != 0u) { --spin; goto L_B3_spin; } goto L_B3_again; } else goto L_B4;
+        if(sure >= 2u)
+        {
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 3, 38u);
+            {
+                unsigned tw0_0, tw0_1, tw0_2, tw0_3;
+                const unsigned tb0 = static_cast<unsigned>(R.r56);
+                if constexpr(kFlat)
+                {
+                    const unsigned* tp = ctx.cols->table + tb0;
+                    tw0_0 = __ldg(tp + 0);
+                    tw0_1 = __ldg(tp + 1);
+                    tw0_2 = __ldg(tp + 2);
+                    tw0_3 = __ldg(tp + 3);
+                }
+                else
+                {
+                    tw0_0 = table_load<unsigned>(*ctx.cols, tb0 + 0u);
+                    tw0_1 = table_load<unsigned>(*ctx.cols, tb0 + 1u);
+                    tw0_2 = table_load<unsigned>(*ctx.cols, tb0 + 2u);
+                    tw0_3 = table_load<unsigned>(*ctx.cols, tb0 + 3u);
+                }
+                R.r57 = static_cast<float>(bitcast<float>(tw0_0));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r58 = static_cast<float>(bitcast<float>(tw0_1));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
+                R.r59 = static_cast<float>(bitcast<float>(tw0_2));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
+                R.r60 = static_cast<float>(bitcast<float>(tw0_3));
+                R.r61 = static_cast<float>(static_cast<float>(static_cast<float>(R.r57) - static_cast<float>(R.r46)));
+                R.r62 = static_cast<float>(static_cast<float>(static_cast<float>(R.r58) - static_cast<float>(R.r47)));
+                R.r63 = static_cast<float>(static_cast<float>(static_cast<float>(R.r59) - static_cast<float>(R.r48)));
+                R.r64 = static_cast<float>((0x0.0p+0f));
+                R.r64 = static_cast<float>(op_fma(R.r61, R.r42, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r62, R.r43, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r63, R.r44, R.r64));
+                R.r65 = static_cast<float>(static_cast<float>(-static_cast<float>(R.r64)));
+                R.r66 = static_cast<float>(op_fma(R.r65, R.r42, R.r61));
+                R.r67 = static_cast<float>(op_fma(R.r65, R.r43, R.r62));
+                R.r68 = static_cast<float>(op_fma(R.r65, R.r44, R.r63));
+                R.r69 = static_cast<float>((0x0.0p+0f));
+                R.r69 = static_cast<float>(op_fma(R.r66, R.r66, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r67, R.r67, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
+                R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
+                R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
+                if(R.r71)
+                {
+                    R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
+                    R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
+                    R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
+                    R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
+                    R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
+                    R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
+                    R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
+                    R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+                }
+                R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
+                R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
+            }
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 3, 38u);
+            {
+                unsigned tw0_0, tw0_1, tw0_2, tw0_3;
+                const unsigned tb0 = static_cast<unsigned>(R.r56);
+                if constexpr(kFlat)
+                {
+                    const unsigned* tp = ctx.cols->table + tb0;
+                    tw0_0 = __ldg(tp + 0);
+                    tw0_1 = __ldg(tp + 1);
+                    tw0_2 = __ldg(tp + 2);
+                    tw0_3 = __ldg(tp + 3);
+                }
+                else
+                {
+                    tw0_0 = table_load<unsigned>(*ctx.cols, tb0 + 0u);
+                    tw0_1 = table_load<unsigned>(*ctx.cols, tb0 + 1u);
+                    tw0_2 = table_load<unsigned>(*ctx.cols, tb0 + 2u);
+                    tw0_3 = table_load<unsigned>(*ctx.cols, tb0 + 3u);
+                }
+                R.r57 = static_cast<float>(bitcast<float>(tw0_0));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r58 = static_cast<float>(bitcast<float>(tw0_1));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
+                R.r59 = static_cast<float>(bitcast<float>(tw0_2));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
+                R.r60 = static_cast<float>(bitcast<float>(tw0_3));
+                R.r61 = static_cast<float>(static_cast<float>(static_cast<float>(R.r57) - static_cast<float>(R.r46)));
+                R.r62 = static_cast<float>(static_cast<float>(static_cast<float>(R.r58) - static_cast<float>(R.r47)));
+                R.r63 = static_cast<float>(static_cast<float>(static_cast<float>(R.r59) - static_cast<float>(R.r48)));
+                R.r64 = static_cast<float>((0x0.0p+0f));
+                R.r64 = static_cast<float>(op_fma(R.r61, R.r42, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r62, R.r43, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r63, R.r44, R.r64));
+                R.r65 = static_cast<float>(static_cast<float>(-static_cast<float>(R.r64)));
+                R.r66 = static_cast<float>(op_fma(R.r65, R.r42, R.r61));
+                R.r67 = static_cast<float>(op_fma(R.r65, R.r43, R.r62));
+                R.r68 = static_cast<float>(op_fma(R.r65, R.r44, R.r63));
+                R.r69 = static_cast<float>((0x0.0p+0f));
+                R.r69 = static_cast<float>(op_fma(R.r66, R.r66, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r67, R.r67, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
+                R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
+                R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
+                if(R.r71)
+                {
+                    R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
+                    R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
+                    R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
+                    R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
+                    R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
+                    R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
+                    R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
+                    R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+                }
+                R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
+                R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
+            }
+            sure -= 2u;
+        }
+        left += sure;
+        while(left)
+        {
+            fresh = false;
+            if constexpr(kProf) count_block(ctx, 3, 38u);
+            {
+                unsigned tw0_0, tw0_1, tw0_2, tw0_3;
+                const unsigned tb0 = static_cast<unsigned>(R.r56);
+                if constexpr(kFlat)
+                {
+                    const unsigned* tp = ctx.cols->table + tb0;
+                    tw0_0 = __ldg(tp + 0);
+                    tw0_1 = __ldg(tp + 1);
+                    tw0_2 = __ldg(tp + 2);
+                    tw0_3 = __ldg(tp + 3);
+                }
+                else
+                {
+                    tw0_0 = table_load<unsigned>(*ctx.cols, tb0 + 0u);
+                    tw0_1 = table_load<unsigned>(*ctx.cols, tb0 + 1u);
+                    tw0_2 = table_load<unsigned>(*ctx.cols, tb0 + 2u);
+                    tw0_3 = table_load<unsigned>(*ctx.cols, tb0 + 3u);
+                }
+                R.r57 = static_cast<float>(bitcast<float>(tw0_0));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r58 = static_cast<float>(bitcast<float>(tw0_1));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x2ull))));
+                R.r59 = static_cast<float>(bitcast<float>(tw0_2));
+                R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x3ull))));
+                R.r60 = static_cast<float>(bitcast<float>(tw0_3));
+                R.r61 = static_cast<float>(static_cast<float>(static_cast<float>(R.r57) - static_cast<float>(R.r46)));
+                R.r62 = static_cast<float>(static_cast<float>(static_cast<float>(R.r58) - static_cast<float>(R.r47)));
+                R.r63 = static_cast<float>(static_cast<float>(static_cast<float>(R.r59) - static_cast<float>(R.r48)));
+                R.r64 = static_cast<float>((0x0.0p+0f));
+                R.r64 = static_cast<float>(op_fma(R.r61, R.r42, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r62, R.r43, R.r64));
+                R.r64 = static_cast<float>(op_fma(R.r63, R.r44, R.r64));
+                R.r65 = static_cast<float>(static_cast<float>(-static_cast<float>(R.r64)));
+                R.r66 = static_cast<float>(op_fma(R.r65, R.r42, R.r61));
+                R.r67 = static_cast<float>(op_fma(R.r65, R.r43, R.r62));
+                R.r68 = static_cast<float>(op_fma(R.r65, R.r44, R.r63));
+                R.r69 = static_cast<float>((0x0.0p+0f));
+                R.r69 = static_cast<float>(op_fma(R.r66, R.r66, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r67, R.r67, R.r69));
+                R.r69 = static_cast<float>(op_fma(R.r68, R.r68, R.r69));
+                R.r70 = static_cast<float>(op_fma(R.r60, R.r60, (-(R.r69))));
+                R.r71 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r70) >= static_cast<float>((0x0.0p+0f))));
+                if(R.r71)
+                {
+                    R.r70 = static_cast<float>(op_max<float>(static_cast<float>(R.r70), static_cast<float>((0x0.0p+0f))));
+                    R.r72 = static_cast<float>(op_sqrt(static_cast<float>(R.r70)));
+                    R.r73 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) - static_cast<float>(R.r72)));
+                    R.r74 = static_cast<float>(static_cast<float>(static_cast<float>(R.r64) + static_cast<float>(R.r72)));
+                    R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(R.r73) > static_cast<float>((0x1.9999980000000p-5f))));
+                    R.r75 = static_cast<float>(((R.r33) ? (R.r73) : (R.r74)));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) > static_cast<float>((0x1.9999980000000p-5f)))));
+                    R.r71 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r71) && static_cast<unsigned int>(static_cast<float>(R.r75) < static_cast<float>(R.r53))));
+                    R.r53 = static_cast<float>(((R.r71) ? (R.r75) : (R.r53)));
+                    R.r54 = static_cast<unsigned int>(((R.r71) ? (R.r55) : (R.r54)));
+                }
+                R.r55 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r55) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+                R.r56 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r56) + static_cast<unsigned int>(((unsigned int)0x8ull))));
+                R.r33 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r55) < static_cast<unsigned int>(R.r13)));
+            }
+            --left;
+            if(!(R.r33)) goto L_B3_out;
+        }
+        if(spin) { spin = 0u; --budget; } else budget = 0u;
+        goto L_B3_again;
+    L_B3_out:
+        if(spin) { spin = left; --budget; } else budget = left;
+        goto L_B4;
     L_B4: // shade
         fresh = false;
         if constexpr(kProf) count_block(ctx, 4, 2u);
