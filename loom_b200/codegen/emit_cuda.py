@@ -224,6 +224,125 @@ OP_COST = {"div": 10, "mod": 20, "sqrt": 9, "rsqrt": 18, "sin": 60, "cos": 60}
 SINK_MIN_COST = 12
 
 
+# Selects of 64-bit integers: instructions of the predicated arm, at most.
+ARM_MAX = 4
+PTX_OP = {"add": "add.u64", "sub": "sub.u64", "mul": "mul.lo.u64", "band": "and.b64", "bor": "or.b64", "bxor": "xor.b64"}
+
+
+def predicated_ptx(arm):
+    """PTX of the instructions of an arm under predicate p, the last one's
+    result in %0, and the registers it reads in operand order (from %2); a
+    product that only the next sum reads becomes a mad.  None: not of plain
+    64-bit integer operations."""
+    value: Dict[int, str] = {}  # register -> its operand or temporary
+    regs: List[int] = []
+
+    def operand(a):
+        if a.is_literal:
+            return f"{a.bits & 0xFFFFFFFFFFFFFFFF:#x}"
+        if a.reg not in value:
+            value[a.reg] = f"%{2 + len(regs)}"
+            regs.append(a.reg)
+        return value[a.reg]
+
+    text = []
+    skip = False
+    for j, x in enumerate(arm):
+        if x.op not in PTX_OP or x.optype[0] not in ("u64", "i64") or any(a.type != x.optype[0] for a in x.args + [x.dst]):
+            return None
+        if skip:
+            skip = False
+            continue
+        nxt = arm[j + 1] if j + 1 < len(arm) else None
+        fused = (
+            x.op == "mul" and nxt is not None and nxt.op == "add"
+            and [not a.is_literal and a.reg == x.dst.reg for a in nxt.args] == [True, False]
+            and (nxt.dst.reg == x.dst.reg or not any(x.dst.reg in y.reads() for y in arm[j + 2 :]))
+            and all(a.type == nxt.optype[0] for a in nxt.args + [nxt.dst]) and nxt.optype[0] in ("u64", "i64")
+        )
+        args = [operand(a) for a in x.args]
+        last = x
+        if fused:
+            args.append(operand(nxt.args[1]))
+            last, skip = nxt, True
+        end = last is arm[-1]
+        dst = "%0" if end else f"t{j}"
+        text.append(f"@p {'mad.lo.u64' if fused else PTX_OP[x.op]} {dst}, {', '.join(args)};")
+        value[last.dst.reg] = dst
+    return " ".join(text), regs
+
+
+def select_arms(instrs, live_out, storage) -> Dict[int, tuple]:
+    """Selects of 64-bit integers whose operands are computed for them alone:
+    {position of the cmov: (positions of the arm that runs in line, positions
+    of the arm predicated over its result, whether that is the second
+    value)}.  A 64-bit select costs two instructions on the ALU pipe, which
+    bounds integer loops; with one arm predicated there is none (Collatz, a
+    warp's iteration with all lanes busy: 17.2 -> 13.2 cycles)."""
+    n = len(instrs)
+    reach: Dict[int, int] = {}  # register -> position of its last definition
+    uses: Dict[int, List[tuple]] = {}  # definition -> [(position, operand)]
+    for p, ins in enumerate(instrs):
+        if isinstance(ins, Compute):
+            for i, a in enumerate(ins.args):
+                if not a.is_literal and a.reg in reach:
+                    uses.setdefault(reach[a.reg], []).append((p, i))
+            reach[ins.dst.reg] = p
+        else:
+            for r in ins.reads():
+                if r in reach:
+                    uses.setdefault(reach[r], []).append((p, 0))
+    kept = {reach[r] for r in live_out if r in reach}
+    out: Dict[int, tuple] = {}
+    taken = set()
+    for q, sel in enumerate(instrs):
+        if not isinstance(sel, Compute) or sel.op != "cmov" or sel.dst.type not in ("u64", "i64"):
+            continue
+        arms = []
+        for side in (1, 2):
+            arm: set = set()
+            grown = True
+            while grown:
+                grown = False
+                for p in range(q):
+                    if p in arm or p in taken or p in kept or not isinstance(instrs[p], Compute):
+                        continue
+                    if instrs[p].op in OP_COST or instrs[p].op in ("assert_fp", "tab", "cmov"):
+                        continue
+                    u = uses.get(p, [])
+                    if u and all(x == (q, side) or x[0] in arm for x in u):
+                        arm.add(p)
+                        grown = True
+            arms.append(sorted(arm))
+        # the arm with the products is predicated (the multiply pipe is not
+        # the ALU's), the other one runs in line
+        muls = [sum(instrs[p].op == "mul" for p in arm) for arm in arms]
+        pick = 0 if muls[0] >= muls[1] else 1
+        both = arms[0] + arms[1]
+        if not arms[pick] or len(arms[pick]) > ARM_MAX or predicated_ptx([instrs[p] for p in arms[pick]]) is None:
+            continue
+        if instrs[arms[pick][-1]].dst != sel.args[1 + pick] or any(not a.is_literal and a.type != sel.dst.type for a in sel.args[1:]):
+            continue
+        # they move down to the select: nothing in between may change what
+        # they read, or touch what they write
+        ok = all(storage[r] in ("u64", "i64") for p in arms[pick] for r in instrs[p].reads() + instrs[p].writes())
+        for p in both:
+            for m in range(p + 1, q):
+                if m in both or not isinstance(instrs[m], Compute):
+                    continue
+                d = instrs[m].dst.reg
+                if d in instrs[p].reads() or d == instrs[p].dst.reg:
+                    ok = False
+        regs = [{instrs[p].dst.reg for p in arm} for arm in arms]
+        # ... and the arm in line, which runs first, nothing the other reads
+        line = {instrs[p].dst.reg for p in arms[1 - pick]}
+        ok = ok and not line & set(predicated_ptx([instrs[p] for p in arms[pick]])[1])
+        if ok and not (sel.args[0].is_literal or sel.args[0].reg in regs[0] | regs[1]):
+            out[q] = (arms[1 - pick], arms[pick], pick == 1)
+            taken |= set(both) | {q}
+    return out
+
+
 def guarded_region(instrs, live_out, fixed):
     """Work of a block that only matters while a condition register holds
     true: (position of the instruction that sets the register, positions of
@@ -387,6 +506,13 @@ class Lowering:
             return f"static_cast<{ct}>({cv(0, t)} {ARITH[op]} {cv(1, t)})"
         if op in BITS:
             return f"static_cast<{ct}>({cv(0, t)} {BITS[op]} {cv(1, t)})"
+        if op in ("eq", "ne") and t in ("u64", "i64"):
+            # against a literal below 2^32: one three-input logic operation
+            # on the halves that sets the predicate, instead of a compare of
+            # each half (the ALU pipe takes two cycles for either)
+            for i, lit in ((0, ins.args[1]), (1, ins.args[0])):
+                if lit.is_literal and not ins.args[i].is_literal and lit.value() in range(1 << 32):
+                    return f"{'' if op == 'ne' else '!'}op_differs({cv(i, 'u64')}, {lit.value():#x}u)"
         if op in CMP:
             return f"static_cast<bool>({cv(0, t)} {CMP[op]} {cv(1, t)})"
         if op in LOGIC:
@@ -472,6 +598,22 @@ class Lowering:
         def emit(pos: int, indent: str) -> List[str]:
             out = []
             ins = instrs[pos]
+            if pos in arms:
+                # one arm in line, the other predicated over its result
+                line, asm, inverted = arms[pos]
+                for p in line:
+                    out.append(indent + self.write(instrs[p].dst, self.expr(instrs[p])))
+                ct = CTYPE[ins.dst.type]
+                c = f"static_cast<unsigned>(static_cast<bool>({self.read(ins.args[0])}))"
+                out.append(indent + "{")
+                out.append(indent + f"    unsigned long long v = static_cast<unsigned long long>({self.read(ins.args[1 if inverted else 2])});")
+                text, regs = predicated_ptx([instrs[p] for p in asm])
+                ops = ", ".join([f'"r"({c})'] + [f'"l"({self.rname(r)})' for r in regs])
+                out.append(indent + f'    asm("{{.reg .pred p; .reg .u64 t<{len(asm) + 1}>; setp.{"eq" if inverted else "ne"}.u32 p, %1, 0; {text}}}"')
+                out.append(indent + f'        : "+l"(v) : {ops});')
+                out.append(indent + "    " + self.write(ins.dst, f"static_cast<{ct}>(v)"))
+                out.append(indent + "}")
+                return out
             if pos in rows:
                 base, dist = rows[pos]
                 out.append(indent + f"const unsigned tb{pos} = static_cast<unsigned>({base});")
@@ -493,11 +635,14 @@ class Lowering:
             return out
 
         todo = [p for p, ins in enumerate(instrs) if isinstance(ins, Compute)]
+        arms = select_arms(instrs, live_out, {i: r.storage for i, r in self.regs.items()}) if live_out is not None else {}
+        in_arm = {p for a, b, _ in arms.values() for p in a + b}
+        todo = [p for p in todo if p not in in_arm]
         out = []
         inner = indent + "    " if rows else indent
         for pos in rows:
             out.append(inner + f"unsigned {', '.join(f'tw{pos}_{d}' for d in rows[pos][1])};")
-        fixed = set(rows) | set(member)
+        fixed = set(rows) | set(member) | set(arms) | in_arm
         sink = guarded_region(instrs, live_out, fixed) if live_out is not None else None
         if sink:
             cond, inside = sink

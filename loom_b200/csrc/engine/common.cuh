@@ -146,6 +146,13 @@ loop_more_ne(const T i, const T n, const unsigned most)
     return loop_more<U>(static_cast<U>(n) - static_cast<U>(i) - 1u, most);
 }
 
+/// Whether v differs from a 32-bit literal.
+__device__ __forceinline__ bool
+op_differs(const unsigned long long v, const unsigned lit)
+{
+    return ((static_cast<unsigned>(v) ^ lit) | static_cast<unsigned>(v >> 32)) != 0u;
+}
+
 __device__ __forceinline__ float op_abs(float v) { return fabsf(v); }
 __device__ __forceinline__ double op_abs(double v) { return fabs(v); }
 __device__ __forceinline__ int op_abs(int v) { return v < 0 ? -v : v; }

@@ -144,81 +144,105 @@ struct K
             if constexpr(kProf) count_block(ctx, 1, 8u);
             R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
             R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            {
+                unsigned long long v = static_cast<unsigned long long>(R.r5);
+                asm("{.reg .pred p; .reg .u64 t<3>; setp.ne.u32 p, %1, 0; @p mad.lo.u64 %0, %2, 0x3, 0x1;}"
+                    : "+l"(v) : "r"(static_cast<unsigned>(static_cast<bool>(R.r4))), "l"(R.r1));
+                R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
+            }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
             R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
             R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            {
+                unsigned long long v = static_cast<unsigned long long>(R.r5);
+                asm("{.reg .pred p; .reg .u64 t<3>; setp.ne.u32 p, %1, 0; @p mad.lo.u64 %0, %2, 0x3, 0x1;}"
+                    : "+l"(v) : "r"(static_cast<unsigned>(static_cast<bool>(R.r4))), "l"(R.r1));
+                R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
+            }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
             R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
             R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            {
+                unsigned long long v = static_cast<unsigned long long>(R.r5);
+                asm("{.reg .pred p; .reg .u64 t<3>; setp.ne.u32 p, %1, 0; @p mad.lo.u64 %0, %2, 0x3, 0x1;}"
+                    : "+l"(v) : "r"(static_cast<unsigned>(static_cast<bool>(R.r4))), "l"(R.r1));
+                R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
+            }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
             R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
             R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            {
+                unsigned long long v = static_cast<unsigned long long>(R.r5);
+                asm("{.reg .pred p; .reg .u64 t<3>; setp.ne.u32 p, %1, 0; @p mad.lo.u64 %0, %2, 0x3, 0x1;}"
+                    : "+l"(v) : "r"(static_cast<unsigned>(static_cast<bool>(R.r4))), "l"(R.r1));
+                R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
+            }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
             R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
             R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            {
+                unsigned long long v = static_cast<unsigned long long>(R.r5);
+                asm("{.reg .pred p; .reg .u64 t<3>; setp.ne.u32 p, %1, 0; @p mad.lo.u64 %0, %2, 0x3, 0x1;}"
+                    : "+l"(v) : "r"(static_cast<unsigned>(static_cast<bool>(R.r4))), "l"(R.r1));
+                R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
+            }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
             R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
             R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            {
+                unsigned long long v = static_cast<unsigned long long>(R.r5);
+                asm("{.reg .pred p; .reg .u64 t<3>; setp.ne.u32 p, %1, 0; @p mad.lo.u64 %0, %2, 0x3, 0x1;}"
+                    : "+l"(v) : "r"(static_cast<unsigned>(static_cast<bool>(R.r4))), "l"(R.r1));
+                R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
+            }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
             R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
             R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            {
+                unsigned long long v = static_cast<unsigned long long>(R.r5);
+                asm("{.reg .pred p; .reg .u64 t<3>; setp.ne.u32 p, %1, 0; @p mad.lo.u64 %0, %2, 0x3, 0x1;}"
+                    : "+l"(v) : "r"(static_cast<unsigned>(static_cast<bool>(R.r4))), "l"(R.r1));
+                R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
+            }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
             R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
             R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            {
+                unsigned long long v = static_cast<unsigned long long>(R.r5);
+                asm("{.reg .pred p; .reg .u64 t<3>; setp.ne.u32 p, %1, 0; @p mad.lo.u64 %0, %2, 0x3, 0x1;}"
+                    : "+l"(v) : "r"(static_cast<unsigned>(static_cast<bool>(R.r4))), "l"(R.r1));
+                R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
+            }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
             if(!(R.r3)) goto L_HALT;
             left -= 8u;
         }
@@ -228,11 +252,14 @@ struct K
             if constexpr(kProf) count_block(ctx, 1, 8u);
             R.r4 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) & static_cast<unsigned long long>(((unsigned long long)0x1ull))));
             R.r5 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) >> static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(((unsigned long long)0x3ull))));
-            R.r6 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r6) + static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r1 = static_cast<unsigned long long>(((R.r4) ? (R.r6) : (R.r5)));
+            {
+                unsigned long long v = static_cast<unsigned long long>(R.r5);
+                asm("{.reg .pred p; .reg .u64 t<3>; setp.ne.u32 p, %1, 0; @p mad.lo.u64 %0, %2, 0x3, 0x1;}"
+                    : "+l"(v) : "r"(static_cast<unsigned>(static_cast<bool>(R.r4))), "l"(R.r1));
+                R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
+            }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(static_cast<bool>(static_cast<unsigned long long>(R.r1) != static_cast<unsigned long long>(((unsigned long long)0x1ull))));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
             --left;
             if(!(R.r3)) goto L_HALT;
         }
