@@ -433,6 +433,15 @@ def guarded_region(instrs, live_out, fixed):
     return best
 
 
+# Selections among constants by one index: from this many on they become
+# 128-bit loads from one row of constant memory.  A chain of compares and
+# selects costs some 4 ALU instructions per value and entry count of 5 (Loom's
+# path tracers fetch a box side's 12 coordinates so on every test); lanes that
+# traverse together read one row.  A 384x384 window of Loom's pt_const 53.9 ->
+# 51.4 ms.
+SCT_MIN = 3
+
+
 class Lowering:
     def __init__(self, k: Kernel):
         self.k = k
@@ -589,15 +598,61 @@ class Lowering:
                 member[p] = (first, d)
         return rows, member
 
-    def body(self, instrs, indent: str, live_out=None) -> List[str]:
+    def constant_rows(self, instrs):
+        """Selections among constants (`sct`) by one index: {position of the
+        first: (index operand, entries, positions)} of every SCT_MIN or more
+        of them on an index that does not change in between, with the same
+        number of 4-byte entries."""
+        groups: Dict[tuple, List[int]] = {}
+        version: Dict[int, int] = {}
+        for p, ins in enumerate(instrs):
+            if not isinstance(ins, Compute):
+                continue
+            a = ins.args[0] if ins.args else None
+            if (
+                ins.op == "sct" and not a.is_literal and a.type in ("u8", "u16", "u32", "u64")
+                and len(ins.consts) >= 3 and all(TYPE_BYTES[c.type] == 4 for c in ins.consts)
+            ):
+                groups.setdefault((a.reg, version.get(a.reg, 0), len(ins.consts)), []).append(p)
+            version[ins.dst.reg] = version.get(ins.dst.reg, 0) + 1
+        return {ps[0]: (instrs[ps[0]].args[0], n, ps) for (_, _, n), ps in groups.items() if len(ps) >= SCT_MIN}
+
+    def constant_tables(self, blk) -> List[str]:
+        """Definitions of a block's constant rows: an entry's values side by
+        side, padded to whole 16-byte words."""
+        out = []
+        for first, (_, n, ps) in self.constant_rows(blk.instrs).items():
+            rows = []
+            for i in range(n):
+                words = [f"{blk.instrs[p].consts[i].bits & 0xFFFFFFFF:#x}u" for p in ps]
+                words += ["0u"] * (-len(words) % 4)
+                rows += ["{" + ", ".join(words[j : j + 4]) + "}" for j in range(0, len(words), 4)]
+            out.append(f"__constant__ uint4 kSct{blk.idx}_{first}[{len(rows)}] = {{{', '.join(rows)}}};")
+        return out
+
+    def body(self, instrs, indent: str, live_out=None, block: int = 0) -> List[str]:
         """The instructions of a block (without its terminator).  `live_out`:
         registers read after them, which allows work that only a condition
         needs to move behind it."""
         rows, member = self.table_rows(instrs)
 
+        sct = self.constant_rows(instrs)
+        sct_of = {p: (first, j) for first, (_, _, ps) in sct.items() for j, p in enumerate(ps)}
+
         def emit(pos: int, indent: str) -> List[str]:
             out = []
             ins = instrs[pos]
+            if pos in sct:
+                idx, n, ps = sct[pos]
+                width = (len(ps) + 3) // 4
+                ct = CTYPE[idx.type]
+                out.append(indent + f"const uint4* sp{pos} = kSct{block}_{pos} + {width}u * static_cast<unsigned>(op_min<{ct}>({self.read(idx)}, {n - 1}));")
+                out.extend(indent + f"const uint4 sv{pos}_{j} = sp{pos}[{j}];" for j in range(width))
+            if pos in sct_of:
+                first, j = sct_of[pos]
+                (t, _) = ins.optype
+                out.append(indent + self.write(ins.dst, f"bitcast<{CTYPE[t]}>(sv{first}_{j // 4}.{'xyzw'[j % 4]})"))
+                return out
             if pos in arms:
                 # one arm in line, the other predicated over its result
                 line, asm, inverted = arms[pos]
@@ -639,10 +694,10 @@ class Lowering:
         in_arm = {p for a, b, _ in arms.values() for p in a + b}
         todo = [p for p in todo if p not in in_arm]
         out = []
-        inner = indent + "    " if rows else indent
+        inner = indent + "    " if rows or sct else indent
         for pos in rows:
             out.append(inner + f"unsigned {', '.join(f'tw{pos}_{d}' for d in rows[pos][1])};")
-        fixed = set(rows) | set(member) | set(arms) | in_arm
+        fixed = set(rows) | set(member) | set(sct_of) | set(arms) | in_arm
         sink = guarded_region(instrs, live_out, fixed) if live_out is not None else None
         if sink:
             cond, inside = sink
@@ -658,7 +713,7 @@ class Lowering:
             todo = [p for p in todo if p > cond and p not in inside]
         for p in todo:
             out.extend(emit(p, inner))
-        if rows:  # a scope of their own: labels of other blocks are jumped to past them
+        if rows or sct:  # a scope of their own: labels of other blocks are jumped to past them
             out = [indent + "{"] + out + [indent + "}"]
         return out
 
@@ -804,6 +859,8 @@ def generate(k: Kernel) -> str:
     heavy = {b for b in range(nb) if quorum[b] > 0}
     w(f"__constant__ unsigned kQuorumTab[{nb}] = {{{', '.join(map(str, quorum))}}};")
     w(f"__constant__ unsigned kRankTab[{nb}] = {{{', '.join(map(str, k.rpo_ranks()))}}};")
+    for blk in k.blocks:
+        o.extend(L.constant_tables(blk))
     w("")
     w("struct K")
     w("{")
@@ -996,7 +1053,7 @@ def generate(k: Kernel) -> str:
         if heavy:
             body.append("        fresh = false;")
         body.append(f"        if constexpr(kProf) count_block(ctx, {b}, {len(blk.instrs)}u);")
-        body.extend(L.body(blk.instrs, "        ", live_outs[b]))
+        body.extend(L.body(blk.instrs, "        ", live_outs[b], b))
         if copies > 1:
             # iterations until the budget has to be looked at again, run in
             # groups of `copies` with one look at their number per group

@@ -11,6 +11,10 @@ __constant__ unsigned kLiveTab[33] = {8, 48, 84, 148, 140, 140, 132, 160, 148, 1
 __constant__ int kQueueBlock[33] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30, 31, 32};
 __constant__ unsigned kQuorumTab[33] = {26, 28, 6, 0, 0, 0, 0, 0, 0, 0, 0, 5, 0, 0, 0, 0, 3, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 6, 0};
 __constant__ unsigned kRankTab[33] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 22, 23, 18, 19, 20, 21, 24, 25, 26, 27, 28, 29, 30, 31, 32};
+__constant__ uint4 kSct2_0[15] = {{0xbf800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0xbf800000u}, {0xbf800000u, 0xbf800000u, 0xbf800000u, 0xbf800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0xbf800000u}, {0xbf800000u, 0xbf800000u, 0xbf800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0x3f800000u, 0xbf800000u, 0xbf800000u, 0x3f800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0x3f800000u}, {0x3f800000u, 0x3f800000u, 0x3f800000u, 0xbf800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0xbf800000u}, {0x3f800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0xbf800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0xbf800000u}};
+__constant__ uint4 kSct11_0[6] = {{0xbf49af9bu, 0xbf800000u, 0xbf167c69u, 0xbf0abdbfu}, {0xbf800000u, 0x3ea8dab7u, 0u, 0u}, {0xbf0abdbfu, 0xbf800000u, 0x3ea8dab7u, 0x3e04e8a1u}, {0xbf800000u, 0xbeaf1517u, 0u, 0u}, {0x3e04e8a1u, 0xbf800000u, 0xbeaf1517u, 0xbf49af9bu}, {0xbf800000u, 0xbf167c69u, 0u, 0u}};
+__constant__ uint4 kSct31_2[8] = {{0x3f4ccccdu, 0x3f4ccccdu, 0x3f4ccccdu, 0u}, {0x3f800000u, 0x3ecccccdu, 0x3e4ccccdu, 0u}, {0x3e4ccccdu, 0x3f800000u, 0x3ecccccdu, 0u}, {0x3f4ccccdu, 0x3f4ccccdu, 0x3f4ccccdu, 0u}, {0x3e99999au, 0x3ecccccdu, 0x3ecccccdu, 0u}, {0x0u, 0x3e591688u, 0x3f0d9169u, 0u}, {0x0u, 0x3e591688u, 0x3f0d9169u, 0u}, {0x0u, 0x3e591688u, 0x3f0d9169u, 0u}};
+__constant__ uint4 kSct31_8[4] = {{0x3f4ccccdu, 0x3e4ccccdu, 0x3f4ccccdu, 0u}, {0x3f800000u, 0x3f49374cu, 0x3eda9fbfu, 0u}, {0x3f800000u, 0x3f49374cu, 0x3eda9fbfu, 0u}, {0x3f800000u, 0x3f800000u, 0x3f800000u, 0u}};
 
 struct K
 {
@@ -587,36 +591,42 @@ struct K
         --budget;
         fresh = false;
         if constexpr(kProf) count_block(ctx, 2, 31u);
-        R.r28 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.0000000000000p+0f) : ((R.r33) == 1 ? (-0x1.0000000000000p+0f) : ((R.r33) == 2 ? (0x1.0000000000000p+0f) : ((R.r33) == 3 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r29 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.0000000000000p+0f) : ((R.r33) == 1 ? (-0x1.0000000000000p+0f) : ((R.r33) == 2 ? (-0x1.0000000000000p+0f) : ((R.r33) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r30 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (0x1.0000000000000p+0f) : ((R.r33) == 1 ? (0x1.0000000000000p+0f) : ((R.r33) == 2 ? (-0x1.0000000000000p+0f) : ((R.r33) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r34 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (0x1.0000000000000p+0f) : ((R.r33) == 1 ? (-0x1.0000000000000p+0f) : ((R.r33) == 2 ? (0x1.0000000000000p+0f) : ((R.r33) == 3 ? (-0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r35 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.0000000000000p+0f) : ((R.r33) == 1 ? (-0x1.0000000000000p+0f) : ((R.r33) == 2 ? (-0x1.0000000000000p+0f) : ((R.r33) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f))))))));
-        R.r36 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (0x1.0000000000000p+0f) : ((R.r33) == 1 ? (-0x1.0000000000000p+0f) : ((R.r33) == 2 ? (0x1.0000000000000p+0f) : ((R.r33) == 3 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r37 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (0x1.0000000000000p+0f) : ((R.r33) == 1 ? (-0x1.0000000000000p+0f) : ((R.r33) == 2 ? (0x1.0000000000000p+0f) : ((R.r33) == 3 ? (0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r38 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.0000000000000p+0f) : ((R.r33) == 1 ? (0x1.0000000000000p+0f) : ((R.r33) == 2 ? (0x1.0000000000000p+0f) : ((R.r33) == 3 ? (0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r39 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.0000000000000p+0f) : ((R.r33) == 1 ? (-0x1.0000000000000p+0f) : ((R.r33) == 2 ? (0x1.0000000000000p+0f) : ((R.r33) == 3 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r40 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.0000000000000p+0f) : ((R.r33) == 1 ? (-0x1.0000000000000p+0f) : ((R.r33) == 2 ? (0x1.0000000000000p+0f) : ((R.r33) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r41 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.0000000000000p+0f) : ((R.r33) == 1 ? (0x1.0000000000000p+0f) : ((R.r33) == 2 ? (0x1.0000000000000p+0f) : ((R.r33) == 3 ? (0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r42 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.0000000000000p+0f) : ((R.r33) == 1 ? (0x1.0000000000000p+0f) : ((R.r33) == 2 ? (-0x1.0000000000000p+0f) : ((R.r33) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r43 = static_cast<float>(static_cast<float>(static_cast<float>(R.r40) - static_cast<float>(R.r28)));
-        R.r44 = static_cast<float>(static_cast<float>(static_cast<float>(R.r41) - static_cast<float>(R.r29)));
-        R.r45 = static_cast<float>(static_cast<float>(static_cast<float>(R.r42) - static_cast<float>(R.r30)));
-        R.r46 = static_cast<float>(static_cast<float>(static_cast<float>(R.r34) - static_cast<float>(R.r28)));
-        R.r47 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r35)) - static_cast<float>(R.r29)));
-        R.r48 = static_cast<float>(static_cast<float>(static_cast<float>(R.r36) - static_cast<float>(R.r30)));
-        R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r27) * static_cast<float>(R.r47))));
-        R.r50 = static_cast<float>(op_fma(bitcast<float>(R.r7), R.r48, (-(bitcast<float>(R.r49)))));
-        R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r48))));
-        R.r51 = static_cast<float>(op_fma(R.r27, R.r46, (-(bitcast<float>(R.r49)))));
-        R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r46))));
-        R.r52 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r47, (-(bitcast<float>(R.r49)))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r43, R.r50, bitcast<float>(R.r14))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r44, R.r51, bitcast<float>(R.r14))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r45, R.r52, bitcast<float>(R.r14))));
-        R.r10 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r14)))));
-        R.r49 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r10)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        {
+            const uint4* sp0 = kSct2_0 + 3u * static_cast<unsigned>(op_min<unsigned int>(R.r33, 4));
+            const uint4 sv0_0 = sp0[0];
+            const uint4 sv0_1 = sp0[1];
+            const uint4 sv0_2 = sp0[2];
+            R.r28 = static_cast<float>(bitcast<float>(sv0_0.x));
+            R.r29 = static_cast<float>(bitcast<float>(sv0_0.y));
+            R.r30 = static_cast<float>(bitcast<float>(sv0_0.z));
+            R.r34 = static_cast<float>(bitcast<float>(sv0_0.w));
+            R.r35 = bitcast<unsigned int>(static_cast<float>(bitcast<float>(sv0_1.x)));
+            R.r36 = static_cast<float>(bitcast<float>(sv0_1.y));
+            R.r37 = static_cast<float>(bitcast<float>(sv0_1.z));
+            R.r38 = static_cast<float>(bitcast<float>(sv0_1.w));
+            R.r39 = static_cast<float>(bitcast<float>(sv0_2.x));
+            R.r40 = static_cast<float>(bitcast<float>(sv0_2.y));
+            R.r41 = static_cast<float>(bitcast<float>(sv0_2.z));
+            R.r42 = static_cast<float>(bitcast<float>(sv0_2.w));
+            R.r43 = static_cast<float>(static_cast<float>(static_cast<float>(R.r40) - static_cast<float>(R.r28)));
+            R.r44 = static_cast<float>(static_cast<float>(static_cast<float>(R.r41) - static_cast<float>(R.r29)));
+            R.r45 = static_cast<float>(static_cast<float>(static_cast<float>(R.r42) - static_cast<float>(R.r30)));
+            R.r46 = static_cast<float>(static_cast<float>(static_cast<float>(R.r34) - static_cast<float>(R.r28)));
+            R.r47 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r35)) - static_cast<float>(R.r29)));
+            R.r48 = static_cast<float>(static_cast<float>(static_cast<float>(R.r36) - static_cast<float>(R.r30)));
+            R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r27) * static_cast<float>(R.r47))));
+            R.r50 = static_cast<float>(op_fma(bitcast<float>(R.r7), R.r48, (-(bitcast<float>(R.r49)))));
+            R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r48))));
+            R.r51 = static_cast<float>(op_fma(R.r27, R.r46, (-(bitcast<float>(R.r49)))));
+            R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r46))));
+            R.r52 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r47, (-(bitcast<float>(R.r49)))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r43, R.r50, bitcast<float>(R.r14))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r44, R.r51, bitcast<float>(R.r14))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r45, R.r52, bitcast<float>(R.r14))));
+            R.r10 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r14)))));
+            R.r49 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r10)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        }
         if(R.r49) goto L_B3; else goto L_B10;
     L_B3: // isect_quad_l1
         fresh = false;
@@ -754,33 +764,38 @@ struct K
         --budget;
         fresh = false;
         if constexpr(kProf) count_block(ctx, 11, 28u);
-        R.r28 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.935f360000000p-1f) : ((R.r33) == 1 ? (-0x1.157b7e0000000p-1f) : (0x1.09d1420000000p-3f)))));
-        R.r29 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.0000000000000p+0f) : ((R.r33) == 1 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))));
-        R.r30 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.2cf8d20000000p-1f) : ((R.r33) == 1 ? (0x1.51b56e0000000p-2f) : (-0x1.5e2a2e0000000p-2f)))));
-        R.r34 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.157b7e0000000p-1f) : ((R.r33) == 1 ? (0x1.09d1420000000p-3f) : (-0x1.935f360000000p-1f)))));
-        R.r35 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(((R.r33) == 0 ? (-0x1.0000000000000p+0f) : ((R.r33) == 1 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f))))));
-        R.r36 = static_cast<float>(static_cast<float>(((R.r33) == 0 ? (0x1.51b56e0000000p-2f) : ((R.r33) == 1 ? (-0x1.5e2a2e0000000p-2f) : (-0x1.2cf8d20000000p-1f)))));
-        R.r37 = static_cast<float>((-0x1.9999980000000p-2f));
-        R.r38 = static_cast<float>((-0x1.6b0f960000000p-3f));
-        R.r39 = static_cast<float>((-0x1.9999980000000p-3f));
-        R.r34 = static_cast<float>(static_cast<float>(static_cast<float>(R.r34) - static_cast<float>(R.r28)));
-        R.r35 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r35)) - static_cast<float>(R.r29))));
-        R.r36 = static_cast<float>(static_cast<float>(static_cast<float>(R.r36) - static_cast<float>(R.r30)));
-        R.r37 = static_cast<float>(static_cast<float>(static_cast<float>(R.r37) - static_cast<float>(R.r28)));
-        R.r38 = static_cast<float>(static_cast<float>(static_cast<float>(R.r38) - static_cast<float>(R.r29)));
-        R.r39 = static_cast<float>(static_cast<float>(static_cast<float>(R.r39) - static_cast<float>(R.r30)));
-        R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r27) * static_cast<float>(R.r38))));
-        R.r40 = static_cast<float>(op_fma(bitcast<float>(R.r7), R.r39, (-(bitcast<float>(R.r49)))));
-        R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r39))));
-        R.r41 = static_cast<float>(op_fma(R.r27, R.r37, (-(bitcast<float>(R.r49)))));
-        R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r37))));
-        R.r42 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r38, (-(bitcast<float>(R.r49)))));
-        R.r53 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
-        R.r53 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r34, R.r40, bitcast<float>(R.r53))));
-        R.r53 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r35), R.r41, bitcast<float>(R.r53))));
-        R.r53 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r36, R.r42, bitcast<float>(R.r53))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r53)))));
-        R.r49 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r14)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        {
+            const uint4* sp0 = kSct11_0 + 2u * static_cast<unsigned>(op_min<unsigned int>(R.r33, 2));
+            const uint4 sv0_0 = sp0[0];
+            const uint4 sv0_1 = sp0[1];
+            R.r28 = static_cast<float>(bitcast<float>(sv0_0.x));
+            R.r29 = static_cast<float>(bitcast<float>(sv0_0.y));
+            R.r30 = static_cast<float>(bitcast<float>(sv0_0.z));
+            R.r34 = static_cast<float>(bitcast<float>(sv0_0.w));
+            R.r35 = bitcast<unsigned int>(static_cast<float>(bitcast<float>(sv0_1.x)));
+            R.r36 = static_cast<float>(bitcast<float>(sv0_1.y));
+            R.r37 = static_cast<float>((-0x1.9999980000000p-2f));
+            R.r38 = static_cast<float>((-0x1.6b0f960000000p-3f));
+            R.r39 = static_cast<float>((-0x1.9999980000000p-3f));
+            R.r34 = static_cast<float>(static_cast<float>(static_cast<float>(R.r34) - static_cast<float>(R.r28)));
+            R.r35 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r35)) - static_cast<float>(R.r29))));
+            R.r36 = static_cast<float>(static_cast<float>(static_cast<float>(R.r36) - static_cast<float>(R.r30)));
+            R.r37 = static_cast<float>(static_cast<float>(static_cast<float>(R.r37) - static_cast<float>(R.r28)));
+            R.r38 = static_cast<float>(static_cast<float>(static_cast<float>(R.r38) - static_cast<float>(R.r29)));
+            R.r39 = static_cast<float>(static_cast<float>(static_cast<float>(R.r39) - static_cast<float>(R.r30)));
+            R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r27) * static_cast<float>(R.r38))));
+            R.r40 = static_cast<float>(op_fma(bitcast<float>(R.r7), R.r39, (-(bitcast<float>(R.r49)))));
+            R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r39))));
+            R.r41 = static_cast<float>(op_fma(R.r27, R.r37, (-(bitcast<float>(R.r49)))));
+            R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r37))));
+            R.r42 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r38, (-(bitcast<float>(R.r49)))));
+            R.r53 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
+            R.r53 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r34, R.r40, bitcast<float>(R.r53))));
+            R.r53 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r35), R.r41, bitcast<float>(R.r53))));
+            R.r53 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r36, R.r42, bitcast<float>(R.r53))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r53)))));
+            R.r49 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r14)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        }
         if(R.r49) goto L_B12; else goto L_B15;
     L_B12: // isect_triangle_mid1
         fresh = false;
@@ -1025,25 +1040,31 @@ struct K
     L_B31_again:
         fresh = false;
         if constexpr(kProf) count_block(ctx, 31, 20u);
-        R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-        R.r14 = static_cast<unsigned int>(op_min<unsigned int>(static_cast<unsigned int>(R.r32), static_cast<unsigned int>(((unsigned int)0x7ull))));
-        R.r23 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.99999a0000000p-1f) : ((R.r14) == 1 ? (0x1.0000000000000p+0f) : ((R.r14) == 2 ? (0x1.99999a0000000p-3f) : ((R.r14) == 3 ? (0x1.99999a0000000p-1f) : ((R.r14) == 4 ? (0x1.3333340000000p-2f) : ((R.r14) == 5 ? (0x0.0p+0f) : ((R.r14) == 6 ? (0x0.0p+0f) : (0x0.0p+0f))))))))));
-        R.r24 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.99999a0000000p-1f) : ((R.r14) == 1 ? (0x1.99999a0000000p-2f) : ((R.r14) == 2 ? (0x1.0000000000000p+0f) : ((R.r14) == 3 ? (0x1.99999a0000000p-1f) : ((R.r14) == 4 ? (0x1.99999a0000000p-2f) : ((R.r14) == 5 ? (0x1.b22d100000000p-3f) : ((R.r14) == 6 ? (0x1.b22d100000000p-3f) : (0x1.b22d100000000p-3f))))))))));
-        R.r25 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.99999a0000000p-1f) : ((R.r14) == 1 ? (0x1.99999a0000000p-3f) : ((R.r14) == 2 ? (0x1.99999a0000000p-2f) : ((R.r14) == 3 ? (0x1.99999a0000000p-1f) : ((R.r14) == 4 ? (0x1.99999a0000000p-2f) : ((R.r14) == 5 ? (0x1.1b22d20000000p-1f) : ((R.r14) == 6 ? (0x1.1b22d20000000p-1f) : (0x1.1b22d20000000p-1f))))))))));
-        R.r14 = static_cast<unsigned int>(op_max<unsigned int>(static_cast<unsigned int>(R.r32), static_cast<unsigned int>(((unsigned int)0x8ull))));
-        R.r14 = static_cast<unsigned int>(op_min<unsigned int>(static_cast<unsigned int>(R.r14), static_cast<unsigned int>(((unsigned int)0xbull))));
-        R.r14 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r14) - static_cast<unsigned int>(((unsigned int)0x8ull))));
-        R.r28 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.99999a0000000p-1f) : ((R.r14) == 1 ? (0x1.0000000000000p+0f) : ((R.r14) == 2 ? (0x1.0000000000000p+0f) : (0x1.0000000000000p+0f))))));
-        R.r29 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.99999a0000000p-3f) : ((R.r14) == 1 ? (0x1.926e980000000p-1f) : ((R.r14) == 2 ? (0x1.926e980000000p-1f) : (0x1.0000000000000p+0f))))));
-        R.r30 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.99999a0000000p-1f) : ((R.r14) == 1 ? (0x1.b53f7e0000000p-2f) : ((R.r14) == 2 ? (0x1.b53f7e0000000p-2f) : (0x1.0000000000000p+0f))))));
-        R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r32) <= static_cast<unsigned int>(((unsigned int)0x7ull))));
-        R.r23 = static_cast<float>(((R.r14) ? (R.r23) : (R.r28)));
-        R.r24 = static_cast<float>(((R.r14) ? (R.r24) : (R.r29)));
-        R.r25 = static_cast<float>(((R.r14) ? (R.r25) : (R.r30)));
-        R.r2 = static_cast<float>(static_cast<float>(static_cast<float>(R.r2) + static_cast<float>(R.r23)));
-        R.r3 = static_cast<float>(static_cast<float>(static_cast<float>(R.r3) + static_cast<float>(R.r24)));
-        R.r4 = static_cast<float>(static_cast<float>(static_cast<float>(R.r4) + static_cast<float>(R.r25)));
-        R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r17) >= static_cast<unsigned int>(((unsigned int)0x40ull))));
+        {
+            R.r5 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r5) + static_cast<unsigned int>(((unsigned int)0x1ull))));
+            R.r14 = static_cast<unsigned int>(op_min<unsigned int>(static_cast<unsigned int>(R.r32), static_cast<unsigned int>(((unsigned int)0x7ull))));
+            const uint4* sp2 = kSct31_2 + 1u * static_cast<unsigned>(op_min<unsigned int>(R.r14, 7));
+            const uint4 sv2_0 = sp2[0];
+            R.r23 = static_cast<float>(bitcast<float>(sv2_0.x));
+            R.r24 = static_cast<float>(bitcast<float>(sv2_0.y));
+            R.r25 = static_cast<float>(bitcast<float>(sv2_0.z));
+            R.r14 = static_cast<unsigned int>(op_max<unsigned int>(static_cast<unsigned int>(R.r32), static_cast<unsigned int>(((unsigned int)0x8ull))));
+            R.r14 = static_cast<unsigned int>(op_min<unsigned int>(static_cast<unsigned int>(R.r14), static_cast<unsigned int>(((unsigned int)0xbull))));
+            R.r14 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r14) - static_cast<unsigned int>(((unsigned int)0x8ull))));
+            const uint4* sp8 = kSct31_8 + 1u * static_cast<unsigned>(op_min<unsigned int>(R.r14, 3));
+            const uint4 sv8_0 = sp8[0];
+            R.r28 = static_cast<float>(bitcast<float>(sv8_0.x));
+            R.r29 = static_cast<float>(bitcast<float>(sv8_0.y));
+            R.r30 = static_cast<float>(bitcast<float>(sv8_0.z));
+            R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r32) <= static_cast<unsigned int>(((unsigned int)0x7ull))));
+            R.r23 = static_cast<float>(((R.r14) ? (R.r23) : (R.r28)));
+            R.r24 = static_cast<float>(((R.r14) ? (R.r24) : (R.r29)));
+            R.r25 = static_cast<float>(((R.r14) ? (R.r25) : (R.r30)));
+            R.r2 = static_cast<float>(static_cast<float>(static_cast<float>(R.r2) + static_cast<float>(R.r23)));
+            R.r3 = static_cast<float>(static_cast<float>(static_cast<float>(R.r3) + static_cast<float>(R.r24)));
+            R.r4 = static_cast<float>(static_cast<float>(static_cast<float>(R.r4) + static_cast<float>(R.r25)));
+            R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r17) >= static_cast<unsigned int>(((unsigned int)0x40ull))));
+        }
         if(R.r14) goto L_B32; else goto L_B1;
     L_B32: // fin_pixel
         fresh = false;

@@ -11,6 +11,10 @@ __constant__ unsigned kLiveTab[55] = {108, 164, 180, 108, 164, 176, 240, 232, 23
 __constant__ int kQueueBlock[55] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30, 31, 32, 33, 34, 35, 36, 37, 38, 39, 40, 41, 42, 43, 44, 45, 46, 47, 48, 49, 50, 51, 52, 53, 54};
 __constant__ unsigned kQuorumTab[55] = {1, 25, 0, 5, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 1, 0, 15, 0, 10, 0, 12, 0, 3, 16, 0, 0};
 __constant__ unsigned kRankTab[55] = {0, 1, 2, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 34, 35, 30, 31, 32, 33, 36, 37, 38, 39, 40, 41, 42, 43, 46, 49, 53, 52, 51, 50, 54, 11, 7, 44, 45, 10, 6, 9, 8, 3, 4, 5, 47, 48};
+__constant__ uint4 kSct5_0[15] = {{0xbf800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0xbf800000u}, {0xbf800000u, 0xbf800000u, 0xbf800000u, 0xbf800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0xbf800000u}, {0xbf800000u, 0xbf800000u, 0xbf800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0x3f800000u, 0xbf800000u, 0xbf800000u, 0x3f800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0x3f800000u}, {0x3f800000u, 0x3f800000u, 0x3f800000u, 0xbf800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0xbf800000u}, {0x3f800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0xbf800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0xbf800000u}};
+__constant__ uint4 kSct14_0[6] = {{0xbf49af9bu, 0xbf800000u, 0xbf167c69u, 0xbf0abdbfu}, {0xbf800000u, 0x3ea8dab7u, 0u, 0u}, {0xbf0abdbfu, 0xbf800000u, 0x3ea8dab7u, 0x3e04e8a1u}, {0xbf800000u, 0xbeaf1517u, 0u, 0u}, {0x3e04e8a1u, 0xbf800000u, 0xbeaf1517u, 0xbf49af9bu}, {0xbf800000u, 0xbf167c69u, 0u, 0u}};
+__constant__ uint4 kSct36_7[6] = {{0x3f800000u, 0x3f800000u, 0x3f800000u, 0u}, {0x3f800000u, 0x3ecccccdu, 0x3e4ccccdu, 0u}, {0x3e4ccccdu, 0x3f800000u, 0x3ecccccdu, 0u}, {0x3f800000u, 0x3f800000u, 0x3f800000u, 0u}, {0x3f800000u, 0x3f800000u, 0x3f800000u, 0u}, {0x0u, 0x3e591688u, 0x3f0d9169u, 0u}};
+__constant__ uint4 kSct37_0[8] = {{0x0u, 0x3f800000u, 0x0u, 0u}, {0x3f800000u, 0x0u, 0x0u, 0u}, {0xbf800000u, 0x0u, 0x0u, 0u}, {0x0u, 0xbf800000u, 0x0u, 0u}, {0x0u, 0x0u, 0x3f800000u, 0u}, {0xbf6a966cu, 0x3ea1e899u, 0x3e7b6e1cu, 0u}, {0x3f2bbae3u, 0x3ea1e89bu, 0x3f2bbae3u, 0u}, {0x3e7b6e22u, 0x3ea1e89bu, 0xbf6a966au, 0u}};
 
 struct K
 {
@@ -692,36 +696,42 @@ struct K
         --budget;
         fresh = false;
         if constexpr(kProf) count_block(ctx, 5, 31u);
-        R.r36 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.0000000000000p+0f) : ((R.r41) == 1 ? (-0x1.0000000000000p+0f) : ((R.r41) == 2 ? (0x1.0000000000000p+0f) : ((R.r41) == 3 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r37 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.0000000000000p+0f) : ((R.r41) == 1 ? (-0x1.0000000000000p+0f) : ((R.r41) == 2 ? (-0x1.0000000000000p+0f) : ((R.r41) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r38 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (0x1.0000000000000p+0f) : ((R.r41) == 1 ? (0x1.0000000000000p+0f) : ((R.r41) == 2 ? (-0x1.0000000000000p+0f) : ((R.r41) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r42 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (0x1.0000000000000p+0f) : ((R.r41) == 1 ? (-0x1.0000000000000p+0f) : ((R.r41) == 2 ? (0x1.0000000000000p+0f) : ((R.r41) == 3 ? (-0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r43 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.0000000000000p+0f) : ((R.r41) == 1 ? (-0x1.0000000000000p+0f) : ((R.r41) == 2 ? (-0x1.0000000000000p+0f) : ((R.r41) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f))))))));
-        R.r44 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(((R.r41) == 0 ? (0x1.0000000000000p+0f) : ((R.r41) == 1 ? (-0x1.0000000000000p+0f) : ((R.r41) == 2 ? (0x1.0000000000000p+0f) : ((R.r41) == 3 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f))))))));
-        R.r45 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (0x1.0000000000000p+0f) : ((R.r41) == 1 ? (-0x1.0000000000000p+0f) : ((R.r41) == 2 ? (0x1.0000000000000p+0f) : ((R.r41) == 3 ? (0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r46 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.0000000000000p+0f) : ((R.r41) == 1 ? (0x1.0000000000000p+0f) : ((R.r41) == 2 ? (0x1.0000000000000p+0f) : ((R.r41) == 3 ? (0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r47 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.0000000000000p+0f) : ((R.r41) == 1 ? (-0x1.0000000000000p+0f) : ((R.r41) == 2 ? (0x1.0000000000000p+0f) : ((R.r41) == 3 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r48 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.0000000000000p+0f) : ((R.r41) == 1 ? (-0x1.0000000000000p+0f) : ((R.r41) == 2 ? (0x1.0000000000000p+0f) : ((R.r41) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f))))))));
-        R.r49 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.0000000000000p+0f) : ((R.r41) == 1 ? (0x1.0000000000000p+0f) : ((R.r41) == 2 ? (0x1.0000000000000p+0f) : ((R.r41) == 3 ? (0x1.0000000000000p+0f) : (0x1.0000000000000p+0f))))))));
-        R.r50 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.0000000000000p+0f) : ((R.r41) == 1 ? (0x1.0000000000000p+0f) : ((R.r41) == 2 ? (-0x1.0000000000000p+0f) : ((R.r41) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r51 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r48)) - static_cast<float>(R.r36)));
-        R.r52 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r49)) - static_cast<float>(R.r37)));
-        R.r53 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r50) - static_cast<float>(R.r38))));
-        R.r54 = static_cast<float>(static_cast<float>(static_cast<float>(R.r42) - static_cast<float>(R.r36)));
-        R.r55 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r43)) - static_cast<float>(R.r37)));
-        R.r56 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r44)) - static_cast<float>(R.r38)));
-        R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r35) * static_cast<float>(R.r55))));
-        R.r58 = static_cast<float>(op_fma(bitcast<float>(R.r7), R.r56, (-(bitcast<float>(R.r57)))));
-        R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r56))));
-        R.r59 = static_cast<float>(op_fma(R.r35, R.r54, (-(bitcast<float>(R.r57)))));
-        R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r54))));
-        R.r60 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r55, (-(bitcast<float>(R.r57)))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r51, R.r58, bitcast<float>(R.r14))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r52, R.r59, bitcast<float>(R.r14))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r53), R.r60, bitcast<float>(R.r14))));
-        R.r8 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r14)))));
-        R.r57 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r8)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        {
+            const uint4* sp0 = kSct5_0 + 3u * static_cast<unsigned>(op_min<unsigned int>(R.r41, 4));
+            const uint4 sv0_0 = sp0[0];
+            const uint4 sv0_1 = sp0[1];
+            const uint4 sv0_2 = sp0[2];
+            R.r36 = static_cast<float>(bitcast<float>(sv0_0.x));
+            R.r37 = static_cast<float>(bitcast<float>(sv0_0.y));
+            R.r38 = static_cast<float>(bitcast<float>(sv0_0.z));
+            R.r42 = static_cast<float>(bitcast<float>(sv0_0.w));
+            R.r43 = bitcast<unsigned int>(static_cast<float>(bitcast<float>(sv0_1.x)));
+            R.r44 = bitcast<unsigned int>(static_cast<float>(bitcast<float>(sv0_1.y)));
+            R.r45 = static_cast<float>(bitcast<float>(sv0_1.z));
+            R.r46 = static_cast<float>(bitcast<float>(sv0_1.w));
+            R.r47 = static_cast<float>(bitcast<float>(sv0_2.x));
+            R.r48 = bitcast<unsigned int>(static_cast<float>(bitcast<float>(sv0_2.y)));
+            R.r49 = bitcast<unsigned int>(static_cast<float>(bitcast<float>(sv0_2.z)));
+            R.r50 = static_cast<float>(bitcast<float>(sv0_2.w));
+            R.r51 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r48)) - static_cast<float>(R.r36)));
+            R.r52 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r49)) - static_cast<float>(R.r37)));
+            R.r53 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r50) - static_cast<float>(R.r38))));
+            R.r54 = static_cast<float>(static_cast<float>(static_cast<float>(R.r42) - static_cast<float>(R.r36)));
+            R.r55 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r43)) - static_cast<float>(R.r37)));
+            R.r56 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r44)) - static_cast<float>(R.r38)));
+            R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r35) * static_cast<float>(R.r55))));
+            R.r58 = static_cast<float>(op_fma(bitcast<float>(R.r7), R.r56, (-(bitcast<float>(R.r57)))));
+            R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r56))));
+            R.r59 = static_cast<float>(op_fma(R.r35, R.r54, (-(bitcast<float>(R.r57)))));
+            R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r54))));
+            R.r60 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r55, (-(bitcast<float>(R.r57)))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r51, R.r58, bitcast<float>(R.r14))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r52, R.r59, bitcast<float>(R.r14))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r53), R.r60, bitcast<float>(R.r14))));
+            R.r8 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r14)))));
+            R.r57 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r8)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        }
         if(R.r57) goto L_B6; else goto L_B13;
     L_B6: // isect_quad_l1
         fresh = false;
@@ -857,33 +867,38 @@ struct K
         --budget;
         fresh = false;
         if constexpr(kProf) count_block(ctx, 14, 28u);
-        R.r36 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.935f360000000p-1f) : ((R.r41) == 1 ? (-0x1.157b7e0000000p-1f) : (0x1.09d1420000000p-3f)))));
-        R.r37 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.0000000000000p+0f) : ((R.r41) == 1 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))));
-        R.r38 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.2cf8d20000000p-1f) : ((R.r41) == 1 ? (0x1.51b56e0000000p-2f) : (-0x1.5e2a2e0000000p-2f)))));
-        R.r42 = static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.157b7e0000000p-1f) : ((R.r41) == 1 ? (0x1.09d1420000000p-3f) : (-0x1.935f360000000p-1f)))));
-        R.r43 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(((R.r41) == 0 ? (-0x1.0000000000000p+0f) : ((R.r41) == 1 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f))))));
-        R.r44 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(((R.r41) == 0 ? (0x1.51b56e0000000p-2f) : ((R.r41) == 1 ? (-0x1.5e2a2e0000000p-2f) : (-0x1.2cf8d20000000p-1f))))));
-        R.r45 = static_cast<float>((-0x1.9999980000000p-2f));
-        R.r46 = static_cast<float>((-0x1.6b0f960000000p-3f));
-        R.r47 = static_cast<float>((-0x1.9999980000000p-3f));
-        R.r42 = static_cast<float>(static_cast<float>(static_cast<float>(R.r42) - static_cast<float>(R.r36)));
-        R.r43 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r43)) - static_cast<float>(R.r37))));
-        R.r44 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r44)) - static_cast<float>(R.r38))));
-        R.r45 = static_cast<float>(static_cast<float>(static_cast<float>(R.r45) - static_cast<float>(R.r36)));
-        R.r46 = static_cast<float>(static_cast<float>(static_cast<float>(R.r46) - static_cast<float>(R.r37)));
-        R.r47 = static_cast<float>(static_cast<float>(static_cast<float>(R.r47) - static_cast<float>(R.r38)));
-        R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r35) * static_cast<float>(R.r46))));
-        R.r48 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r7), R.r47, (-(bitcast<float>(R.r57))))));
-        R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r47))));
-        R.r49 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r35, R.r45, (-(bitcast<float>(R.r57))))));
-        R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r45))));
-        R.r50 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r46, (-(bitcast<float>(R.r57)))));
-        R.r61 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
-        R.r61 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r42, bitcast<float>(R.r48), bitcast<float>(R.r61))));
-        R.r61 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r43), bitcast<float>(R.r49), bitcast<float>(R.r61))));
-        R.r61 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r44), R.r50, bitcast<float>(R.r61))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r61)))));
-        R.r57 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r14)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        {
+            const uint4* sp0 = kSct14_0 + 2u * static_cast<unsigned>(op_min<unsigned int>(R.r41, 2));
+            const uint4 sv0_0 = sp0[0];
+            const uint4 sv0_1 = sp0[1];
+            R.r36 = static_cast<float>(bitcast<float>(sv0_0.x));
+            R.r37 = static_cast<float>(bitcast<float>(sv0_0.y));
+            R.r38 = static_cast<float>(bitcast<float>(sv0_0.z));
+            R.r42 = static_cast<float>(bitcast<float>(sv0_0.w));
+            R.r43 = bitcast<unsigned int>(static_cast<float>(bitcast<float>(sv0_1.x)));
+            R.r44 = bitcast<unsigned int>(static_cast<float>(bitcast<float>(sv0_1.y)));
+            R.r45 = static_cast<float>((-0x1.9999980000000p-2f));
+            R.r46 = static_cast<float>((-0x1.6b0f960000000p-3f));
+            R.r47 = static_cast<float>((-0x1.9999980000000p-3f));
+            R.r42 = static_cast<float>(static_cast<float>(static_cast<float>(R.r42) - static_cast<float>(R.r36)));
+            R.r43 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r43)) - static_cast<float>(R.r37))));
+            R.r44 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r44)) - static_cast<float>(R.r38))));
+            R.r45 = static_cast<float>(static_cast<float>(static_cast<float>(R.r45) - static_cast<float>(R.r36)));
+            R.r46 = static_cast<float>(static_cast<float>(static_cast<float>(R.r46) - static_cast<float>(R.r37)));
+            R.r47 = static_cast<float>(static_cast<float>(static_cast<float>(R.r47) - static_cast<float>(R.r38)));
+            R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r35) * static_cast<float>(R.r46))));
+            R.r48 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r7), R.r47, (-(bitcast<float>(R.r57))))));
+            R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r47))));
+            R.r49 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r35, R.r45, (-(bitcast<float>(R.r57))))));
+            R.r57 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r45))));
+            R.r50 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r46, (-(bitcast<float>(R.r57)))));
+            R.r61 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
+            R.r61 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r42, bitcast<float>(R.r48), bitcast<float>(R.r61))));
+            R.r61 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r43), bitcast<float>(R.r49), bitcast<float>(R.r61))));
+            R.r61 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r44), R.r50, bitcast<float>(R.r61))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r61)))));
+            R.r57 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r14)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        }
         if(R.r57) goto L_B15; else goto L_B18;
     L_B15: // isect_triangle_mid1
         fresh = false;
@@ -1149,36 +1164,40 @@ struct K
     L_B36: // set_materials
         fresh = false;
         if constexpr(kProf) count_block(ctx, 36, 31u);
-        R.r36 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r39)));
-        R.r37 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r39)));
-        R.r38 = static_cast<float>(static_cast<float>(static_cast<float>(R.r35) * static_cast<float>(R.r39)));
-        R.r22 = static_cast<float>(static_cast<float>(static_cast<float>(R.r22) + static_cast<float>(R.r36)));
-        R.r23 = static_cast<float>(static_cast<float>(static_cast<float>(R.r23) + static_cast<float>(R.r37)));
-        R.r24 = static_cast<float>(static_cast<float>(static_cast<float>(R.r24) + static_cast<float>(R.r38)));
-        R.r14 = static_cast<unsigned int>(op_min<unsigned int>(static_cast<unsigned int>(R.r40), static_cast<unsigned int>(((unsigned int)0x5ull))));
-        R.r31 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.0000000000000p+0f) : ((R.r14) == 1 ? (0x1.0000000000000p+0f) : ((R.r14) == 2 ? (0x1.99999a0000000p-3f) : ((R.r14) == 3 ? (0x1.0000000000000p+0f) : ((R.r14) == 4 ? (0x1.0000000000000p+0f) : (0x0.0p+0f))))))));
-        R.r32 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.0000000000000p+0f) : ((R.r14) == 1 ? (0x1.99999a0000000p-2f) : ((R.r14) == 2 ? (0x1.0000000000000p+0f) : ((R.r14) == 3 ? (0x1.0000000000000p+0f) : ((R.r14) == 4 ? (0x1.0000000000000p+0f) : (0x1.b22d100000000p-3f))))))));
-        R.r33 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.0000000000000p+0f) : ((R.r14) == 1 ? (0x1.99999a0000000p-3f) : ((R.r14) == 2 ? (0x1.99999a0000000p-2f) : ((R.r14) == 3 ? (0x1.0000000000000p+0f) : ((R.r14) == 4 ? (0x1.0000000000000p+0f) : (0x1.1b22d20000000p-1f))))))));
-        R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0x8ull))));
-        R.r31 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r31)));
-        R.r32 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r32)));
-        R.r33 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r33)));
-        R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0x9ull))));
-        R.r14 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r14) || static_cast<unsigned int>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0xaull)))));
-        R.r31 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r31)));
-        R.r32 = static_cast<float>(((R.r14) ? ((0x1.a76c8c0000000p-1f)) : (R.r32)));
-        R.r33 = static_cast<float>(((R.r14) ? ((0x1.12f1aa0000000p-1f)) : (R.r33)));
-        R.r62 = static_cast<float>((0x0.0p+0f));
-        R.r63 = static_cast<float>((0x1.0000000000000p+0f));
-        R.r64 = static_cast<float>((0x0.0p+0f));
-        R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0xaull))));
-        R.r14 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r14) || static_cast<unsigned int>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0xbull)))));
-        R.r8 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0x8ull))));
-        R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r8) || static_cast<unsigned int>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0x9ull)))));
-        R.r41 = static_cast<unsigned int>(((unsigned int)0x0ull));
-        R.r41 = static_cast<unsigned int>(((R.r14) ? (((unsigned int)0x1ull)) : (R.r41)));
-        R.r9 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r40) - static_cast<unsigned int>(((unsigned int)0x6ull))));
-        R.r41 = static_cast<unsigned int>(((R.r8) ? (R.r9) : (R.r41)));
+        {
+            R.r36 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r39)));
+            R.r37 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r39)));
+            R.r38 = static_cast<float>(static_cast<float>(static_cast<float>(R.r35) * static_cast<float>(R.r39)));
+            R.r22 = static_cast<float>(static_cast<float>(static_cast<float>(R.r22) + static_cast<float>(R.r36)));
+            R.r23 = static_cast<float>(static_cast<float>(static_cast<float>(R.r23) + static_cast<float>(R.r37)));
+            R.r24 = static_cast<float>(static_cast<float>(static_cast<float>(R.r24) + static_cast<float>(R.r38)));
+            R.r14 = static_cast<unsigned int>(op_min<unsigned int>(static_cast<unsigned int>(R.r40), static_cast<unsigned int>(((unsigned int)0x5ull))));
+            const uint4* sp7 = kSct36_7 + 1u * static_cast<unsigned>(op_min<unsigned int>(R.r14, 5));
+            const uint4 sv7_0 = sp7[0];
+            R.r31 = static_cast<float>(bitcast<float>(sv7_0.x));
+            R.r32 = static_cast<float>(bitcast<float>(sv7_0.y));
+            R.r33 = static_cast<float>(bitcast<float>(sv7_0.z));
+            R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0x8ull))));
+            R.r31 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r31)));
+            R.r32 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r32)));
+            R.r33 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r33)));
+            R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0x9ull))));
+            R.r14 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r14) || static_cast<unsigned int>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0xaull)))));
+            R.r31 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r31)));
+            R.r32 = static_cast<float>(((R.r14) ? ((0x1.a76c8c0000000p-1f)) : (R.r32)));
+            R.r33 = static_cast<float>(((R.r14) ? ((0x1.12f1aa0000000p-1f)) : (R.r33)));
+            R.r62 = static_cast<float>((0x0.0p+0f));
+            R.r63 = static_cast<float>((0x1.0000000000000p+0f));
+            R.r64 = static_cast<float>((0x0.0p+0f));
+            R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0xaull))));
+            R.r14 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r14) || static_cast<unsigned int>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0xbull)))));
+            R.r8 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0x8ull))));
+            R.r8 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r8) || static_cast<unsigned int>(static_cast<unsigned int>(R.r40) == static_cast<unsigned int>(((unsigned int)0x9ull)))));
+            R.r41 = static_cast<unsigned int>(((unsigned int)0x0ull));
+            R.r41 = static_cast<unsigned int>(((R.r14) ? (((unsigned int)0x1ull)) : (R.r41)));
+            R.r9 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r40) - static_cast<unsigned int>(((unsigned int)0x6ull))));
+            R.r41 = static_cast<unsigned int>(((R.r8) ? (R.r9) : (R.r41)));
+        }
         switch(R.r41) {
         case 0: goto L_B37;
         case 1: goto L_B38;
@@ -1189,9 +1208,13 @@ struct K
     L_B37: // set_polygon_normal
         fresh = false;
         if constexpr(kProf) count_block(ctx, 37, 4u);
-        R.r65 = static_cast<float>(static_cast<float>(((R.r40) == 0 ? (0x0.0p+0f) : ((R.r40) == 1 ? (0x1.0000000000000p+0f) : ((R.r40) == 2 ? (-0x1.0000000000000p+0f) : ((R.r40) == 3 ? (0x0.0p+0f) : ((R.r40) == 4 ? (0x0.0p+0f) : ((R.r40) == 5 ? (-0x1.d52cd80000000p-1f) : ((R.r40) == 6 ? (0x1.5775c60000000p-1f) : (0x1.f6dc440000000p-3f))))))))));
-        R.r66 = static_cast<float>(static_cast<float>(((R.r40) == 0 ? (0x1.0000000000000p+0f) : ((R.r40) == 1 ? (0x0.0p+0f) : ((R.r40) == 2 ? (0x0.0p+0f) : ((R.r40) == 3 ? (-0x1.0000000000000p+0f) : ((R.r40) == 4 ? (0x0.0p+0f) : ((R.r40) == 5 ? (0x1.43d1320000000p-2f) : ((R.r40) == 6 ? (0x1.43d1360000000p-2f) : (0x1.43d1360000000p-2f))))))))));
-        R.r67 = static_cast<float>(static_cast<float>(((R.r40) == 0 ? (0x0.0p+0f) : ((R.r40) == 1 ? (0x0.0p+0f) : ((R.r40) == 2 ? (0x0.0p+0f) : ((R.r40) == 3 ? (0x0.0p+0f) : ((R.r40) == 4 ? (0x1.0000000000000p+0f) : ((R.r40) == 5 ? (0x1.f6dc380000000p-3f) : ((R.r40) == 6 ? (0x1.5775c60000000p-1f) : (-0x1.d52cd40000000p-1f))))))))));
+        {
+            const uint4* sp0 = kSct37_0 + 1u * static_cast<unsigned>(op_min<unsigned int>(R.r40, 7));
+            const uint4 sv0_0 = sp0[0];
+            R.r65 = static_cast<float>(bitcast<float>(sv0_0.x));
+            R.r66 = static_cast<float>(bitcast<float>(sv0_0.y));
+            R.r67 = static_cast<float>(bitcast<float>(sv0_0.z));
+        }
         goto L_B41;
     L_B38: // set_disk_normal
         fresh = false;

@@ -11,6 +11,10 @@ __constant__ unsigned kLiveTab[44] = {64, 124, 76, 120, 132, 196, 188, 188, 180,
 __constant__ int kQueueBlock[44] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 23, 24, 25, 26, 27, 28, 29, 30, 31, 32, 33, 34, 35, 36, 37, 38, 39, 40, 41, 42, 43};
 __constant__ unsigned kQuorumTab[44] = {8, 26, 9, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 3, 0, 0, 0, 0, 0, 13, 0, 0};
 __constant__ unsigned kRankTab[44] = {0, 1, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 25, 26, 21, 22, 23, 24, 27, 28, 29, 30, 31, 32, 33, 34, 35, 38, 42, 41, 40, 39, 43, 2, 36, 37};
+__constant__ uint4 kSct4_0[15] = {{0xbf800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0xbf800000u}, {0xbf800000u, 0xbf800000u, 0xbf800000u, 0xbf800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0xbf800000u}, {0xbf800000u, 0xbf800000u, 0xbf800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0x3f800000u, 0xbf800000u, 0xbf800000u, 0x3f800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0x3f800000u}, {0x3f800000u, 0x3f800000u, 0x3f800000u, 0xbf800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0xbf800000u}, {0x3f800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0x3f800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0xbf800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0x3f800000u}, {0xbf800000u, 0xbf800000u, 0x3f800000u, 0xbf800000u}};
+__constant__ uint4 kSct13_0[6] = {{0xbf49af9bu, 0xbf800000u, 0xbf167c69u, 0xbf0abdbfu}, {0xbf800000u, 0x3ea8dab7u, 0u, 0u}, {0xbf0abdbfu, 0xbf800000u, 0x3ea8dab7u, 0x3e04e8a1u}, {0xbf800000u, 0xbeaf1517u, 0u, 0u}, {0x3e04e8a1u, 0xbf800000u, 0xbeaf1517u, 0xbf49af9bu}, {0xbf800000u, 0xbf167c69u, 0u, 0u}};
+__constant__ uint4 kSct35_7[6] = {{0x3f800000u, 0x3f800000u, 0x3f800000u, 0u}, {0x3f800000u, 0x3ecccccdu, 0x3e4ccccdu, 0u}, {0x3e4ccccdu, 0x3f800000u, 0x3ecccccdu, 0u}, {0x3f800000u, 0x3f800000u, 0x3f800000u, 0u}, {0x3f800000u, 0x3f800000u, 0x3f800000u, 0u}, {0x0u, 0x3e591688u, 0x3f0d9169u, 0u}};
+__constant__ uint4 kSct36_0[8] = {{0x0u, 0x3f800000u, 0x0u, 0u}, {0x3f800000u, 0x0u, 0x0u, 0u}, {0xbf800000u, 0x0u, 0x0u, 0u}, {0x0u, 0xbf800000u, 0x0u, 0u}, {0x0u, 0x0u, 0x3f800000u, 0u}, {0xbf6a966cu, 0x3ea1e899u, 0x3e7b6e1cu, 0u}, {0x3f2bbae3u, 0x3ea1e89bu, 0x3f2bbae3u, 0u}, {0x3e7b6e22u, 0x3ea1e89bu, 0xbf6a966au, 0u}};
 
 struct K
 {
@@ -641,36 +645,42 @@ struct K
         --budget;
         fresh = false;
         if constexpr(kProf) count_block(ctx, 4, 31u);
-        R.r33 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.0000000000000p+0f) : ((R.r38) == 1 ? (-0x1.0000000000000p+0f) : ((R.r38) == 2 ? (0x1.0000000000000p+0f) : ((R.r38) == 3 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r34 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.0000000000000p+0f) : ((R.r38) == 1 ? (-0x1.0000000000000p+0f) : ((R.r38) == 2 ? (-0x1.0000000000000p+0f) : ((R.r38) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r35 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (0x1.0000000000000p+0f) : ((R.r38) == 1 ? (0x1.0000000000000p+0f) : ((R.r38) == 2 ? (-0x1.0000000000000p+0f) : ((R.r38) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r39 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (0x1.0000000000000p+0f) : ((R.r38) == 1 ? (-0x1.0000000000000p+0f) : ((R.r38) == 2 ? (0x1.0000000000000p+0f) : ((R.r38) == 3 ? (-0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r40 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.0000000000000p+0f) : ((R.r38) == 1 ? (-0x1.0000000000000p+0f) : ((R.r38) == 2 ? (-0x1.0000000000000p+0f) : ((R.r38) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f))))))));
-        R.r41 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (0x1.0000000000000p+0f) : ((R.r38) == 1 ? (-0x1.0000000000000p+0f) : ((R.r38) == 2 ? (0x1.0000000000000p+0f) : ((R.r38) == 3 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r42 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (0x1.0000000000000p+0f) : ((R.r38) == 1 ? (-0x1.0000000000000p+0f) : ((R.r38) == 2 ? (0x1.0000000000000p+0f) : ((R.r38) == 3 ? (0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r43 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.0000000000000p+0f) : ((R.r38) == 1 ? (0x1.0000000000000p+0f) : ((R.r38) == 2 ? (0x1.0000000000000p+0f) : ((R.r38) == 3 ? (0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r44 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.0000000000000p+0f) : ((R.r38) == 1 ? (-0x1.0000000000000p+0f) : ((R.r38) == 2 ? (0x1.0000000000000p+0f) : ((R.r38) == 3 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r45 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.0000000000000p+0f) : ((R.r38) == 1 ? (-0x1.0000000000000p+0f) : ((R.r38) == 2 ? (0x1.0000000000000p+0f) : ((R.r38) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r46 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.0000000000000p+0f) : ((R.r38) == 1 ? (0x1.0000000000000p+0f) : ((R.r38) == 2 ? (0x1.0000000000000p+0f) : ((R.r38) == 3 ? (0x1.0000000000000p+0f) : (0x1.0000000000000p+0f)))))));
-        R.r47 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.0000000000000p+0f) : ((R.r38) == 1 ? (0x1.0000000000000p+0f) : ((R.r38) == 2 ? (-0x1.0000000000000p+0f) : ((R.r38) == 3 ? (0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))))));
-        R.r48 = static_cast<float>(static_cast<float>(static_cast<float>(R.r45) - static_cast<float>(R.r33)));
-        R.r49 = static_cast<float>(static_cast<float>(static_cast<float>(R.r46) - static_cast<float>(R.r34)));
-        R.r50 = static_cast<float>(static_cast<float>(static_cast<float>(R.r47) - static_cast<float>(R.r35)));
-        R.r51 = static_cast<float>(static_cast<float>(static_cast<float>(R.r39) - static_cast<float>(R.r33)));
-        R.r52 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r40)) - static_cast<float>(R.r34)));
-        R.r53 = static_cast<float>(static_cast<float>(static_cast<float>(R.r41) - static_cast<float>(R.r35)));
-        R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r32) * static_cast<float>(R.r52))));
-        R.r55 = static_cast<float>(op_fma(bitcast<float>(R.r7), R.r53, (-(bitcast<float>(R.r54)))));
-        R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r53))));
-        R.r56 = static_cast<float>(op_fma(R.r32, R.r51, (-(bitcast<float>(R.r54)))));
-        R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r51))));
-        R.r57 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r52, (-(bitcast<float>(R.r54)))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r48, R.r55, bitcast<float>(R.r14))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r49, R.r56, bitcast<float>(R.r14))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r50, R.r57, bitcast<float>(R.r14))));
-        R.r10 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r14)))));
-        R.r54 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r10)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        {
+            const uint4* sp0 = kSct4_0 + 3u * static_cast<unsigned>(op_min<unsigned int>(R.r38, 4));
+            const uint4 sv0_0 = sp0[0];
+            const uint4 sv0_1 = sp0[1];
+            const uint4 sv0_2 = sp0[2];
+            R.r33 = static_cast<float>(bitcast<float>(sv0_0.x));
+            R.r34 = static_cast<float>(bitcast<float>(sv0_0.y));
+            R.r35 = static_cast<float>(bitcast<float>(sv0_0.z));
+            R.r39 = static_cast<float>(bitcast<float>(sv0_0.w));
+            R.r40 = bitcast<unsigned int>(static_cast<float>(bitcast<float>(sv0_1.x)));
+            R.r41 = static_cast<float>(bitcast<float>(sv0_1.y));
+            R.r42 = static_cast<float>(bitcast<float>(sv0_1.z));
+            R.r43 = static_cast<float>(bitcast<float>(sv0_1.w));
+            R.r44 = static_cast<float>(bitcast<float>(sv0_2.x));
+            R.r45 = static_cast<float>(bitcast<float>(sv0_2.y));
+            R.r46 = static_cast<float>(bitcast<float>(sv0_2.z));
+            R.r47 = static_cast<float>(bitcast<float>(sv0_2.w));
+            R.r48 = static_cast<float>(static_cast<float>(static_cast<float>(R.r45) - static_cast<float>(R.r33)));
+            R.r49 = static_cast<float>(static_cast<float>(static_cast<float>(R.r46) - static_cast<float>(R.r34)));
+            R.r50 = static_cast<float>(static_cast<float>(static_cast<float>(R.r47) - static_cast<float>(R.r35)));
+            R.r51 = static_cast<float>(static_cast<float>(static_cast<float>(R.r39) - static_cast<float>(R.r33)));
+            R.r52 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r40)) - static_cast<float>(R.r34)));
+            R.r53 = static_cast<float>(static_cast<float>(static_cast<float>(R.r41) - static_cast<float>(R.r35)));
+            R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r32) * static_cast<float>(R.r52))));
+            R.r55 = static_cast<float>(op_fma(bitcast<float>(R.r7), R.r53, (-(bitcast<float>(R.r54)))));
+            R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r53))));
+            R.r56 = static_cast<float>(op_fma(R.r32, R.r51, (-(bitcast<float>(R.r54)))));
+            R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r51))));
+            R.r57 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r52, (-(bitcast<float>(R.r54)))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r48, R.r55, bitcast<float>(R.r14))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r49, R.r56, bitcast<float>(R.r14))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r50, R.r57, bitcast<float>(R.r14))));
+            R.r10 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r14)))));
+            R.r54 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r10)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        }
         if(R.r54) goto L_B5; else goto L_B12;
     L_B5: // isect_quad_l1
         fresh = false;
@@ -806,33 +816,38 @@ struct K
         --budget;
         fresh = false;
         if constexpr(kProf) count_block(ctx, 13, 28u);
-        R.r33 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.935f360000000p-1f) : ((R.r38) == 1 ? (-0x1.157b7e0000000p-1f) : (0x1.09d1420000000p-3f)))));
-        R.r34 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.0000000000000p+0f) : ((R.r38) == 1 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f)))));
-        R.r35 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.2cf8d20000000p-1f) : ((R.r38) == 1 ? (0x1.51b56e0000000p-2f) : (-0x1.5e2a2e0000000p-2f)))));
-        R.r39 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.157b7e0000000p-1f) : ((R.r38) == 1 ? (0x1.09d1420000000p-3f) : (-0x1.935f360000000p-1f)))));
-        R.r40 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(((R.r38) == 0 ? (-0x1.0000000000000p+0f) : ((R.r38) == 1 ? (-0x1.0000000000000p+0f) : (-0x1.0000000000000p+0f))))));
-        R.r41 = static_cast<float>(static_cast<float>(((R.r38) == 0 ? (0x1.51b56e0000000p-2f) : ((R.r38) == 1 ? (-0x1.5e2a2e0000000p-2f) : (-0x1.2cf8d20000000p-1f)))));
-        R.r42 = static_cast<float>((-0x1.9999980000000p-2f));
-        R.r43 = static_cast<float>((-0x1.6b0f960000000p-3f));
-        R.r44 = static_cast<float>((-0x1.9999980000000p-3f));
-        R.r39 = static_cast<float>(static_cast<float>(static_cast<float>(R.r39) - static_cast<float>(R.r33)));
-        R.r40 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r40)) - static_cast<float>(R.r34))));
-        R.r41 = static_cast<float>(static_cast<float>(static_cast<float>(R.r41) - static_cast<float>(R.r35)));
-        R.r42 = static_cast<float>(static_cast<float>(static_cast<float>(R.r42) - static_cast<float>(R.r33)));
-        R.r43 = static_cast<float>(static_cast<float>(static_cast<float>(R.r43) - static_cast<float>(R.r34)));
-        R.r44 = static_cast<float>(static_cast<float>(static_cast<float>(R.r44) - static_cast<float>(R.r35)));
-        R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r32) * static_cast<float>(R.r43))));
-        R.r45 = static_cast<float>(op_fma(bitcast<float>(R.r7), R.r44, (-(bitcast<float>(R.r54)))));
-        R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r44))));
-        R.r46 = static_cast<float>(op_fma(R.r32, R.r42, (-(bitcast<float>(R.r54)))));
-        R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r42))));
-        R.r47 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r43, (-(bitcast<float>(R.r54)))));
-        R.r58 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
-        R.r58 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r39, R.r45, bitcast<float>(R.r58))));
-        R.r58 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r40), R.r46, bitcast<float>(R.r58))));
-        R.r58 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r41, R.r47, bitcast<float>(R.r58))));
-        R.r14 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r58)))));
-        R.r54 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r14)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        {
+            const uint4* sp0 = kSct13_0 + 2u * static_cast<unsigned>(op_min<unsigned int>(R.r38, 2));
+            const uint4 sv0_0 = sp0[0];
+            const uint4 sv0_1 = sp0[1];
+            R.r33 = static_cast<float>(bitcast<float>(sv0_0.x));
+            R.r34 = static_cast<float>(bitcast<float>(sv0_0.y));
+            R.r35 = static_cast<float>(bitcast<float>(sv0_0.z));
+            R.r39 = static_cast<float>(bitcast<float>(sv0_0.w));
+            R.r40 = bitcast<unsigned int>(static_cast<float>(bitcast<float>(sv0_1.x)));
+            R.r41 = static_cast<float>(bitcast<float>(sv0_1.y));
+            R.r42 = static_cast<float>((-0x1.9999980000000p-2f));
+            R.r43 = static_cast<float>((-0x1.6b0f960000000p-3f));
+            R.r44 = static_cast<float>((-0x1.9999980000000p-3f));
+            R.r39 = static_cast<float>(static_cast<float>(static_cast<float>(R.r39) - static_cast<float>(R.r33)));
+            R.r40 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r40)) - static_cast<float>(R.r34))));
+            R.r41 = static_cast<float>(static_cast<float>(static_cast<float>(R.r41) - static_cast<float>(R.r35)));
+            R.r42 = static_cast<float>(static_cast<float>(static_cast<float>(R.r42) - static_cast<float>(R.r33)));
+            R.r43 = static_cast<float>(static_cast<float>(static_cast<float>(R.r43) - static_cast<float>(R.r34)));
+            R.r44 = static_cast<float>(static_cast<float>(static_cast<float>(R.r44) - static_cast<float>(R.r35)));
+            R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(R.r32) * static_cast<float>(R.r43))));
+            R.r45 = static_cast<float>(op_fma(bitcast<float>(R.r7), R.r44, (-(bitcast<float>(R.r54)))));
+            R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r44))));
+            R.r46 = static_cast<float>(op_fma(R.r32, R.r42, (-(bitcast<float>(R.r54)))));
+            R.r54 = bitcast<unsigned int>(static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r42))));
+            R.r47 = static_cast<float>(op_fma(bitcast<float>(R.r6), R.r43, (-(bitcast<float>(R.r54)))));
+            R.r58 = bitcast<unsigned int>(static_cast<float>((0x0.0p+0f)));
+            R.r58 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r39, R.r45, bitcast<float>(R.r58))));
+            R.r58 = bitcast<unsigned int>(static_cast<float>(op_fma(bitcast<float>(R.r40), R.r46, bitcast<float>(R.r58))));
+            R.r58 = bitcast<unsigned int>(static_cast<float>(op_fma(R.r41, R.r47, bitcast<float>(R.r58))));
+            R.r14 = bitcast<unsigned int>(static_cast<float>(op_abs(static_cast<float>(bitcast<float>(R.r58)))));
+            R.r54 = static_cast<unsigned int>(static_cast<bool>(static_cast<float>(bitcast<float>(R.r14)) >= static_cast<float>((0x1.a36e2e0000000p-14f))));
+        }
         if(R.r54) goto L_B14; else goto L_B17;
     L_B14: // isect_triangle_mid1
         fresh = false;
@@ -1093,36 +1108,40 @@ struct K
     L_B35_again:
         fresh = false;
         if constexpr(kProf) count_block(ctx, 35, 31u);
-        R.r33 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r36)));
-        R.r34 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r36)));
-        R.r35 = static_cast<float>(static_cast<float>(static_cast<float>(R.r32) * static_cast<float>(R.r36)));
-        R.r22 = static_cast<float>(static_cast<float>(static_cast<float>(R.r22) + static_cast<float>(R.r33)));
-        R.r23 = static_cast<float>(static_cast<float>(static_cast<float>(R.r23) + static_cast<float>(R.r34)));
-        R.r24 = static_cast<float>(static_cast<float>(static_cast<float>(R.r24) + static_cast<float>(R.r35)));
-        R.r14 = static_cast<unsigned int>(op_min<unsigned int>(static_cast<unsigned int>(R.r37), static_cast<unsigned int>(((unsigned int)0x5ull))));
-        R.r28 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.0000000000000p+0f) : ((R.r14) == 1 ? (0x1.0000000000000p+0f) : ((R.r14) == 2 ? (0x1.99999a0000000p-3f) : ((R.r14) == 3 ? (0x1.0000000000000p+0f) : ((R.r14) == 4 ? (0x1.0000000000000p+0f) : (0x0.0p+0f))))))));
-        R.r29 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.0000000000000p+0f) : ((R.r14) == 1 ? (0x1.99999a0000000p-2f) : ((R.r14) == 2 ? (0x1.0000000000000p+0f) : ((R.r14) == 3 ? (0x1.0000000000000p+0f) : ((R.r14) == 4 ? (0x1.0000000000000p+0f) : (0x1.b22d100000000p-3f))))))));
-        R.r30 = static_cast<float>(static_cast<float>(((R.r14) == 0 ? (0x1.0000000000000p+0f) : ((R.r14) == 1 ? (0x1.99999a0000000p-3f) : ((R.r14) == 2 ? (0x1.99999a0000000p-2f) : ((R.r14) == 3 ? (0x1.0000000000000p+0f) : ((R.r14) == 4 ? (0x1.0000000000000p+0f) : (0x1.1b22d20000000p-1f))))))));
-        R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0x8ull))));
-        R.r28 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r28)));
-        R.r29 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r29)));
-        R.r30 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r30)));
-        R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0x9ull))));
-        R.r14 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r14) || static_cast<unsigned int>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0xaull)))));
-        R.r28 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r28)));
-        R.r29 = static_cast<float>(((R.r14) ? ((0x1.a76c8c0000000p-1f)) : (R.r29)));
-        R.r30 = static_cast<float>(((R.r14) ? ((0x1.12f1aa0000000p-1f)) : (R.r30)));
-        R.r59 = static_cast<float>((0x0.0p+0f));
-        R.r60 = static_cast<float>((0x1.0000000000000p+0f));
-        R.r61 = static_cast<float>((0x0.0p+0f));
-        R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0xaull))));
-        R.r14 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r14) || static_cast<unsigned int>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0xbull)))));
-        R.r10 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0x8ull))));
-        R.r10 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r10) || static_cast<unsigned int>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0x9ull)))));
-        R.r38 = static_cast<unsigned int>(((unsigned int)0x0ull));
-        R.r38 = static_cast<unsigned int>(((R.r14) ? (((unsigned int)0x1ull)) : (R.r38)));
-        R.r11 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r37) - static_cast<unsigned int>(((unsigned int)0x6ull))));
-        R.r38 = static_cast<unsigned int>(((R.r10) ? (R.r11) : (R.r38)));
+        {
+            R.r33 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r6)) * static_cast<float>(R.r36)));
+            R.r34 = static_cast<float>(static_cast<float>(static_cast<float>(bitcast<float>(R.r7)) * static_cast<float>(R.r36)));
+            R.r35 = static_cast<float>(static_cast<float>(static_cast<float>(R.r32) * static_cast<float>(R.r36)));
+            R.r22 = static_cast<float>(static_cast<float>(static_cast<float>(R.r22) + static_cast<float>(R.r33)));
+            R.r23 = static_cast<float>(static_cast<float>(static_cast<float>(R.r23) + static_cast<float>(R.r34)));
+            R.r24 = static_cast<float>(static_cast<float>(static_cast<float>(R.r24) + static_cast<float>(R.r35)));
+            R.r14 = static_cast<unsigned int>(op_min<unsigned int>(static_cast<unsigned int>(R.r37), static_cast<unsigned int>(((unsigned int)0x5ull))));
+            const uint4* sp7 = kSct35_7 + 1u * static_cast<unsigned>(op_min<unsigned int>(R.r14, 5));
+            const uint4 sv7_0 = sp7[0];
+            R.r28 = static_cast<float>(bitcast<float>(sv7_0.x));
+            R.r29 = static_cast<float>(bitcast<float>(sv7_0.y));
+            R.r30 = static_cast<float>(bitcast<float>(sv7_0.z));
+            R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0x8ull))));
+            R.r28 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r28)));
+            R.r29 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r29)));
+            R.r30 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r30)));
+            R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0x9ull))));
+            R.r14 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r14) || static_cast<unsigned int>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0xaull)))));
+            R.r28 = static_cast<float>(((R.r14) ? ((0x1.0000000000000p+0f)) : (R.r28)));
+            R.r29 = static_cast<float>(((R.r14) ? ((0x1.a76c8c0000000p-1f)) : (R.r29)));
+            R.r30 = static_cast<float>(((R.r14) ? ((0x1.12f1aa0000000p-1f)) : (R.r30)));
+            R.r59 = static_cast<float>((0x0.0p+0f));
+            R.r60 = static_cast<float>((0x1.0000000000000p+0f));
+            R.r61 = static_cast<float>((0x0.0p+0f));
+            R.r14 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0xaull))));
+            R.r14 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r14) || static_cast<unsigned int>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0xbull)))));
+            R.r10 = static_cast<unsigned int>(static_cast<bool>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0x8ull))));
+            R.r10 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r10) || static_cast<unsigned int>(static_cast<unsigned int>(R.r37) == static_cast<unsigned int>(((unsigned int)0x9ull)))));
+            R.r38 = static_cast<unsigned int>(((unsigned int)0x0ull));
+            R.r38 = static_cast<unsigned int>(((R.r14) ? (((unsigned int)0x1ull)) : (R.r38)));
+            R.r11 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r37) - static_cast<unsigned int>(((unsigned int)0x6ull))));
+            R.r38 = static_cast<unsigned int>(((R.r10) ? (R.r11) : (R.r38)));
+        }
         switch(R.r38) {
         case 0: goto L_B36;
         case 1: goto L_B37;
@@ -1133,9 +1152,13 @@ struct K
     L_B36: // set_polygon_normal
         fresh = false;
         if constexpr(kProf) count_block(ctx, 36, 4u);
-        R.r62 = static_cast<float>(static_cast<float>(((R.r37) == 0 ? (0x0.0p+0f) : ((R.r37) == 1 ? (0x1.0000000000000p+0f) : ((R.r37) == 2 ? (-0x1.0000000000000p+0f) : ((R.r37) == 3 ? (0x0.0p+0f) : ((R.r37) == 4 ? (0x0.0p+0f) : ((R.r37) == 5 ? (-0x1.d52cd80000000p-1f) : ((R.r37) == 6 ? (0x1.5775c60000000p-1f) : (0x1.f6dc440000000p-3f))))))))));
-        R.r63 = static_cast<float>(static_cast<float>(((R.r37) == 0 ? (0x1.0000000000000p+0f) : ((R.r37) == 1 ? (0x0.0p+0f) : ((R.r37) == 2 ? (0x0.0p+0f) : ((R.r37) == 3 ? (-0x1.0000000000000p+0f) : ((R.r37) == 4 ? (0x0.0p+0f) : ((R.r37) == 5 ? (0x1.43d1320000000p-2f) : ((R.r37) == 6 ? (0x1.43d1360000000p-2f) : (0x1.43d1360000000p-2f))))))))));
-        R.r64 = static_cast<float>(static_cast<float>(((R.r37) == 0 ? (0x0.0p+0f) : ((R.r37) == 1 ? (0x0.0p+0f) : ((R.r37) == 2 ? (0x0.0p+0f) : ((R.r37) == 3 ? (0x0.0p+0f) : ((R.r37) == 4 ? (0x1.0000000000000p+0f) : ((R.r37) == 5 ? (0x1.f6dc380000000p-3f) : ((R.r37) == 6 ? (0x1.5775c60000000p-1f) : (-0x1.d52cd40000000p-1f))))))))));
+        {
+            const uint4* sp0 = kSct36_0 + 1u * static_cast<unsigned>(op_min<unsigned int>(R.r37, 7));
+            const uint4 sv0_0 = sp0[0];
+            R.r62 = static_cast<float>(bitcast<float>(sv0_0.x));
+            R.r63 = static_cast<float>(bitcast<float>(sv0_0.y));
+            R.r64 = static_cast<float>(bitcast<float>(sv0_0.z));
+        }
         goto L_B40;
     L_B37: // set_disk_normal
         fresh = false;
