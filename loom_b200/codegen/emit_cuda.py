@@ -1326,21 +1326,34 @@ def generate(k: Kernel) -> str:
         w(f"    {{{offs}, {t[0]}ull, {t[1]}u, {t[2]}u}},")
     w("};")
     w("")
+    flat = "true" if table_rows else "false"
+    w("const void* plain_fn(bool profile, bool flat)")
+    w("{")
+    w("    if(profile) return reinterpret_cast<const void*>(&plain_kernel<K, true, false>);")
+    if table_rows:
+        w("    if(!flat) return reinterpret_cast<const void*>(&plain_kernel<K, false, false>);")
+    w("    (void)flat;")
+    w(f"    return reinterpret_cast<const void*>(&plain_kernel<K, false, {flat}>);")
+    w("}")
+    w("")
     w("cudaError_t launch_plain(const PlainLaunch& a)")
     w("{")
     w("    const unsigned long long grid = (a.n + a.block - 1) / a.block;")
     w("    if(grid == 0) return cudaSuccess;")
-    w("    if(a.profile)")
-    w("        plain_kernel<K, true, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(")
-    w("            a.cols, a.first, a.n, a.max_steps, a.status, a.counters);")
-    if table_rows:
-        w("    else if(!a.cols.table_flat)")
-        w("        plain_kernel<K, false, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(")
-        w("            a.cols, a.first, a.n, a.max_steps, a.status, a.counters);")
-    w("    else")
-    w(f"        plain_kernel<K, false, {'true' if table_rows else 'false'}><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(")
-    w("            a.cols, a.first, a.n, a.max_steps, a.status, a.counters);")
-    w("    return cudaGetLastError();")
+    w("    const void* fn     = plain_fn(a.profile, a.cols.table_flat != 0u);")
+    w("    void*       args[] = {const_cast<Columns*>(&a.cols), const_cast<unsigned long long*>(&a.first),")
+    w("                          const_cast<unsigned long long*>(&a.n), const_cast<unsigned long long*>(&a.max_steps),")
+    w("                          const_cast<unsigned**>(&a.status), const_cast<unsigned long long**>(&a.counters)};")
+    w("    return cudaLaunchKernel(fn, dim3(static_cast<unsigned>(grid)), dim3(a.block), args, 0, a.stream);")
+    w("}")
+    w("")
+    w("// registers of a thread of the plain kernel")
+    w("cudaError_t plain_regs(bool profile, bool flat, int* regs)")
+    w("{")
+    w("    cudaFuncAttributes  at{};")
+    w("    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat));")
+    w("    *regs = at.numRegs;")
+    w("    return e;")
     w("}")
     w("")
     caps = reg_caps(k)
@@ -1409,6 +1422,7 @@ def generate(k: Kernel) -> str:
     w(f"    &loom_b200::k_{name}::kInfo, loom_b200::k_{name}::K::kRowBytes, {nq},")
     w(f"    &loom_b200::k_{name}::launch_plain, &loom_b200::k_{name}::launch_regroup,")
     w(f"    &loom_b200::k_{name}::regroup_occupancy,")
+    w(f"    &loom_b200::k_{name}::plain_regs,")
     w(f"    loom_b200::k_{name}::kQueues, loom_b200::k_{name}::kSegments,")
     w(f"    loom_b200::k_{name}::kRegCaps, {len(caps)}u, loom_b200::k_{name}::K::kMaxStageRow}};")
     return "\n".join(o) + "\n"

@@ -235,17 +235,31 @@ const QueueSegment kSegments[] = {
     {kQOffs0, kQSubs0, kQWidths0, 0ull, 0u, 4u},
 };
 
+const void* plain_fn(bool profile, bool flat)
+{
+    if(profile) return reinterpret_cast<const void*>(&plain_kernel<K, true, false>);
+    (void)flat;
+    return reinterpret_cast<const void*>(&plain_kernel<K, false, false>);
+}
+
 cudaError_t launch_plain(const PlainLaunch& a)
 {
     const unsigned long long grid = (a.n + a.block - 1) / a.block;
     if(grid == 0) return cudaSuccess;
-    if(a.profile)
-        plain_kernel<K, true, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
-            a.cols, a.first, a.n, a.max_steps, a.status, a.counters);
-    else
-        plain_kernel<K, false, false><<<static_cast<unsigned>(grid), a.block, 0, a.stream>>>(
-            a.cols, a.first, a.n, a.max_steps, a.status, a.counters);
-    return cudaGetLastError();
+    const void* fn     = plain_fn(a.profile, a.cols.table_flat != 0u);
+    void*       args[] = {const_cast<Columns*>(&a.cols), const_cast<unsigned long long*>(&a.first),
+                          const_cast<unsigned long long*>(&a.n), const_cast<unsigned long long*>(&a.max_steps),
+                          const_cast<unsigned**>(&a.status), const_cast<unsigned long long**>(&a.counters)};
+    return cudaLaunchKernel(fn, dim3(static_cast<unsigned>(grid)), dim3(a.block), args, 0, a.stream);
+}
+
+// registers of a thread of the plain kernel
+cudaError_t plain_regs(bool profile, bool flat, int* regs)
+{
+    cudaFuncAttributes  at{};
+    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat));
+    *regs = at.numRegs;
+    return e;
 }
 
 const unsigned kRegCaps[] = {64u, 40u, 48u};
@@ -316,5 +330,6 @@ const loom_b200::KernelEntry loom_b200_entry_bool_not_u8 = {
     &loom_b200::k_bool_not_u8::kInfo, loom_b200::k_bool_not_u8::K::kRowBytes, 1,
     &loom_b200::k_bool_not_u8::launch_plain, &loom_b200::k_bool_not_u8::launch_regroup,
     &loom_b200::k_bool_not_u8::regroup_occupancy,
+    &loom_b200::k_bool_not_u8::plain_regs,
     loom_b200::k_bool_not_u8::kQueues, loom_b200::k_bool_not_u8::kSegments,
     loom_b200::k_bool_not_u8::kRegCaps, 3u, loom_b200::k_bool_not_u8::K::kMaxStageRow};

@@ -241,6 +241,7 @@ constexpr unsigned long long kBarrierSpins       = 1ull << 25;
 constexpr unsigned long long kDefaultStateBudget = 8ull << 30; // queue state bytes
 constexpr unsigned           kDefaultPlainBlock  = 256;
 constexpr unsigned           kDefaultRegroupBlock = 256;
+constexpr int                kOneWarpRegs         = 57; // allocated in steps of 8: 65536 / (64 * 32) = 32 warps
 constexpr unsigned           kDefaultUtr         = 16;
 constexpr unsigned           kDefaultPeriod      = 1024;
 constexpr unsigned           kDefaultBurst       = 32;
@@ -289,6 +290,9 @@ struct loom_b200_handle
     RegroupLaunch   graph_key{};
     uint64_t        graph_admit  = 0;
     bool            graph_broken = false; // capture refused: launch directly
+
+    bool     own_block    = true; // the plain engine picks its CTA size
+    unsigned plain_blk[2] = {0, 0}; // its choice, by whether the table is flat (0: not made yet)
 
     loom_b200_stats stats{};
     unsigned        last_grid     = 0;
@@ -375,6 +379,13 @@ grow(void** p, size_t* have, size_t bytes)
     LB_CUDA(cudaMalloc(p, bytes));
     *have = bytes;
     return LOOM_B200_OK;
+}
+
+/// Whether a CTA size asks for one (normalise replaces the others).
+bool
+names_block(const loom_b200_opts& o)
+{
+    return o.block_size != 0 && o.block_size % 32 == 0 && o.block_size <= 1024;
 }
 
 void
@@ -468,6 +479,30 @@ launch_graph(loom_b200_handle* h, const RegroupLaunch& L, uint64_t admit, cudaSt
     }
     LB_CUDA(cudaGraphLaunch(h->graph_exec, stream));
     h->stats.graph_launches += 1;
+    return LOOM_B200_OK;
+}
+
+/// CTA size of a plain launch whose caller named none: the default, or one
+/// warp for a kernel of so many registers (kOneWarpRegs) that the 32 CTAs an
+/// SM can hold are as many warps as its registers can.  The registers of a
+/// CTA come free when its slowest warp ends, and the threads of the large
+/// kernels (path tracers) differ by large factors: 512x512 pixels of Loom's
+/// pt_const 70.0 -> 61.9 ms with CTAs of one warp, a 320x240x16 sphere render
+/// 3.08 -> 2.81 ms; kernels of few registers lose (2^20 Fibonacci threads 24
+/// -> 32 us) as half their warps do not fit.
+int
+plain_block(loom_b200_handle* h, PlainLaunch& L)
+{
+    const bool flat = L.cols.table_flat != 0u;
+    if(L.profile) return LOOM_B200_OK;
+    unsigned& blk = h->plain_blk[flat];
+    if(blk == 0)
+    {
+        int regs = 0;
+        LB_CUDA(h->e->plain_regs(false, flat, &regs));
+        blk = regs >= kOneWarpRegs ? 32u : kDefaultPlainBlock;
+    }
+    L.block = blk;
     return LOOM_B200_OK;
 }
 
@@ -626,8 +661,13 @@ launch(loom_b200_handle* h, const loom_b200_launch& L, cudaStream_t stream, uint
         L.block     = o.block_size;
         L.profile   = o.profile != 0;
         L.stream    = stream;
+        if(h->own_block)
+        {
+            const int rc = plain_block(h, L);
+            if(rc) return rc;
+        }
         LB_CUDA(e.plain(L));
-        h->last_grid = static_cast<unsigned>((n + o.block_size - 1) / o.block_size);
+        h->last_grid = static_cast<unsigned>((n + L.block - 1) / L.block);
         h->plain_threads += n;
     }
     LB_CUDA(cudaEventRecord(h->ev1, stream));
@@ -730,6 +770,8 @@ loom_b200_create(const char*           kernel,
     h->e        = e;
     h->capacity = capacity;
     if(opts) h->opts = *opts;
+    // a regrouping handle's CTA size is the megakernel's
+    h->own_block = h->opts.mode == LOOM_B200_REGROUP || !names_block(h->opts);
     normalise(h->opts);
     auto fail = [&](int rc)
     {
@@ -804,6 +846,7 @@ loom_b200_set_opts(loom_b200_handle* h, const loom_b200_opts* opts)
         if(rc != LOOM_B200_OK && rc != LOOM_B200_ERR_DEVICE) return rc;
     }
     h->opts = *opts;
+    h->own_block = h->opts.mode == LOOM_B200_REGROUP || !names_block(h->opts);
     normalise(h->opts);
     return LOOM_B200_OK;
 }

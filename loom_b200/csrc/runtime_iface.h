@@ -67,6 +67,7 @@ struct KernelEntry
     cudaError_t (*regroup)(const RegroupLaunch&);
     cudaError_t (*regroup_occupancy)(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park,
                                      bool flat, int* ctas_per_sm);
+    cudaError_t (*plain_regs)(bool profile, bool flat, int* regs); // registers per thread of the plain kernel
     const loom_b200_queue_layout* queues;   // num_queues entries
     const QueueSegment*           segments; // num_queues entries
     const unsigned*               reg_caps; // compiled register caps, default first
