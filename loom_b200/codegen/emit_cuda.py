@@ -1327,20 +1327,27 @@ def generate(k: Kernel) -> str:
     w("};")
     w("")
     flat = "true" if table_rows else "false"
-    w("const void* plain_fn(bool profile, bool flat)")
+    w("const void* plain_fn(bool profile, bool flat, unsigned per)")
     w("{")
-    w("    if(profile) return reinterpret_cast<const void*>(&plain_kernel<K, true, false>);")
+    w("    if(profile) return reinterpret_cast<const void*>(&plain_kernel<K, true, false, 1>);")
     if table_rows:
-        w("    if(!flat) return reinterpret_cast<const void*>(&plain_kernel<K, false, false>);")
+        w("    if(!flat) return reinterpret_cast<const void*>(&plain_kernel<K, false, false, 1>);")
+    several = not k.loop_headers() and not table_rows
+    if not several:
+        w("    (void)per;")
+    else:
+        w(f"    if(per > 1u) return reinterpret_cast<const void*>(&plain_kernel<K, false, {flat}, kStraightPer>);")
     w("    (void)flat;")
-    w(f"    return reinterpret_cast<const void*>(&plain_kernel<K, false, {flat}>);")
+    w(f"    return reinterpret_cast<const void*>(&plain_kernel<K, false, {flat}, 1>);")
     w("}")
     w("")
     w("cudaError_t launch_plain(const PlainLaunch& a)")
     w("{")
-    w("    const unsigned long long grid = (a.n + a.block - 1) / a.block;")
+    w("    const bool               flat = a.cols.table_flat != 0u;")
+    w("    const unsigned long long cta  = static_cast<unsigned long long>(a.block) * a.per;")
+    w("    const unsigned long long grid = (a.n + cta - 1) / cta;")
     w("    if(grid == 0) return cudaSuccess;")
-    w("    const void* fn     = plain_fn(a.profile, a.cols.table_flat != 0u);")
+    w("    const void* fn     = plain_fn(a.profile, flat, a.per);")
     w("    void*       args[] = {const_cast<Columns*>(&a.cols), const_cast<unsigned long long*>(&a.first),")
     w("                          const_cast<unsigned long long*>(&a.n), const_cast<unsigned long long*>(&a.max_steps),")
     w("                          const_cast<unsigned**>(&a.status), const_cast<unsigned long long**>(&a.counters)};")
@@ -1351,7 +1358,7 @@ def generate(k: Kernel) -> str:
     w("cudaError_t plain_regs(bool profile, bool flat, int* regs)")
     w("{")
     w("    cudaFuncAttributes  at{};")
-    w("    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat));")
+    w("    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat, 1u));")
     w("    *regs = at.numRegs;")
     w("    return e;")
     w("}")
@@ -1424,7 +1431,7 @@ def generate(k: Kernel) -> str:
     w(f"    &loom_b200::k_{name}::regroup_occupancy,")
     w(f"    &loom_b200::k_{name}::plain_regs,")
     w(f"    loom_b200::k_{name}::kQueues, loom_b200::k_{name}::kSegments,")
-    w(f"    loom_b200::k_{name}::kRegCaps, {len(caps)}u, loom_b200::k_{name}::K::kMaxStageRow}};")
+    w(f"    loom_b200::k_{name}::kRegCaps, {len(caps)}u, loom_b200::k_{name}::K::kMaxStageRow, {"loom_b200::kStraightPer" if several else "1u"}}};")
     return "\n".join(o) + "\n"
 
 

@@ -530,18 +530,21 @@ const QueueSegment kSegments[] = {
     {kQOffs0, kQSubs0, kQWidths0, 0ull, 8u, 16u},
 };
 
-const void* plain_fn(bool profile, bool flat)
+const void* plain_fn(bool profile, bool flat, unsigned per)
 {
-    if(profile) return reinterpret_cast<const void*>(&plain_kernel<K, true, false>);
+    if(profile) return reinterpret_cast<const void*>(&plain_kernel<K, true, false, 1>);
+    if(per > 1u) return reinterpret_cast<const void*>(&plain_kernel<K, false, false, kStraightPer>);
     (void)flat;
-    return reinterpret_cast<const void*>(&plain_kernel<K, false, false>);
+    return reinterpret_cast<const void*>(&plain_kernel<K, false, false, 1>);
 }
 
 cudaError_t launch_plain(const PlainLaunch& a)
 {
-    const unsigned long long grid = (a.n + a.block - 1) / a.block;
+    const bool               flat = a.cols.table_flat != 0u;
+    const unsigned long long cta  = static_cast<unsigned long long>(a.block) * a.per;
+    const unsigned long long grid = (a.n + cta - 1) / cta;
     if(grid == 0) return cudaSuccess;
-    const void* fn     = plain_fn(a.profile, a.cols.table_flat != 0u);
+    const void* fn     = plain_fn(a.profile, flat, a.per);
     void*       args[] = {const_cast<Columns*>(&a.cols), const_cast<unsigned long long*>(&a.first),
                           const_cast<unsigned long long*>(&a.n), const_cast<unsigned long long*>(&a.max_steps),
                           const_cast<unsigned**>(&a.status), const_cast<unsigned long long**>(&a.counters)};
@@ -552,7 +555,7 @@ cudaError_t launch_plain(const PlainLaunch& a)
 cudaError_t plain_regs(bool profile, bool flat, int* regs)
 {
     cudaFuncAttributes  at{};
-    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat));
+    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat, 1u));
     *regs = at.numRegs;
     return e;
 }
@@ -627,4 +630,4 @@ const loom_b200::KernelEntry loom_b200_entry_threefry_u32 = {
     &loom_b200::k_threefry_u32::regroup_occupancy,
     &loom_b200::k_threefry_u32::plain_regs,
     loom_b200::k_threefry_u32::kQueues, loom_b200::k_threefry_u32::kSegments,
-    loom_b200::k_threefry_u32::kRegCaps, 3u, loom_b200::k_threefry_u32::K::kMaxStageRow};
+    loom_b200::k_threefry_u32::kRegCaps, 3u, loom_b200::k_threefry_u32::K::kMaxStageRow, loom_b200::kStraightPer};

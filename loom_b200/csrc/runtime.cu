@@ -241,6 +241,10 @@ constexpr unsigned long long kBarrierSpins       = 1ull << 25;
 constexpr unsigned long long kDefaultStateBudget = 8ull << 30; // queue state bytes
 constexpr unsigned           kDefaultPlainBlock  = 256;
 constexpr unsigned           kDefaultRegroupBlock = 256;
+// Threads per SM from which programs without loops run several Loom threads
+// per CUDA thread: where the GPU is still full of CUDA threads.  2e7 Threefry
+// counters 147 -> 130 us with 4 (2 and 8 a few per cent slower).
+constexpr unsigned long long kStraightFill        = 2048ull * kStraightPer;
 constexpr int                kOneWarpRegs         = 57; // allocated in steps of 8: 65536 / (64 * 32) = 32 warps
 constexpr unsigned           kDefaultUtr         = 16;
 constexpr unsigned           kDefaultPeriod      = 1024;
@@ -660,6 +664,7 @@ launch(loom_b200_handle* h, const loom_b200_launch& L, cudaStream_t stream, uint
         L.counters  = h->d_counters;
         L.block     = o.block_size;
         L.profile   = o.profile != 0;
+        L.per       = n >= kStraightFill * h->sms && o.profile == 0 ? e.per : 1u;
         L.stream    = stream;
         if(h->own_block)
         {
@@ -667,7 +672,8 @@ launch(loom_b200_handle* h, const loom_b200_launch& L, cudaStream_t stream, uint
             if(rc) return rc;
         }
         LB_CUDA(e.plain(L));
-        h->last_grid = static_cast<unsigned>((n + L.block - 1) / L.block);
+        const uint64_t cta = static_cast<uint64_t>(L.block) * L.per;
+        h->last_grid       = static_cast<unsigned>((n + cta - 1) / cta);
         h->plain_threads += n;
     }
     LB_CUDA(cudaEventRecord(h->ev1, stream));

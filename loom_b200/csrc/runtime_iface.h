@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include "engine/plain.cuh"
 #include "engine/regroup.cuh"
 #include "loom_b200.h"
 
@@ -19,6 +20,7 @@ struct PlainLaunch
     unsigned long long* counters;
     unsigned            block;
     bool                profile;
+    unsigned            per; // Loom threads per CUDA thread: 1, or KernelEntry::per
     cudaStream_t        stream;
 };
 
@@ -73,6 +75,7 @@ struct KernelEntry
     const unsigned*               reg_caps; // compiled register caps, default first
     unsigned                      num_reg_caps;
     unsigned                      max_stage_row; // K::kMaxStageRow (bulk_restore staging per entry)
+    unsigned                      per;           // Loom threads per CUDA thread of a large plain launch
 };
 
 /// Whether a launch's table is flat (Columns::table_flat): no table, or one
