@@ -139,6 +139,17 @@ def counted_loop(blk):
     return None
 
 
+def bit_heavy(blk) -> bool:
+    """Whether a long block is mostly shifts and logic, which only the ALU pipe
+    runs, at half the issue rate.  In programs without loops, of which the SM
+    holds warps enough to hide latency, its 32-bit sums then go to the
+    multiply pipe: 2e7 Threefry counters 130 -> 118 us.  In the path tracers,
+    whose serial rounds wait on latency, the longer multiply-add lost: the
+    1024x768x64 render 22.8 -> 23.7 ms."""
+    n = sum(1 for x in blk.instrs if isinstance(x, Compute) and x.op in ("bxor", "bor", "band", "shl", "shr"))
+    return len(blk.instrs) >= LONG_BLOCK_INSTR and 2 * n >= len(blk.instrs)
+
+
 def reg_caps(k: Kernel) -> List[int]:
     """Register caps of the megakernel compiled for `k`, default first."""
     extra = REG_VARIANTS if sum(k.instr_counts()) > REG_VARIANT_MIN_INSTR else SMALL_REG_VARIANTS
@@ -447,6 +458,7 @@ class Lowering:
         self.k = k
         self.pc = k.pc_reg()
         self.regs = {r.idx: r for r in k.regs}
+        self.mad_adds = False
 
     # ------------------------------------------------------------ views
     def rname(self, idx: int) -> str:
@@ -511,6 +523,8 @@ class Lowering:
             return f"static_cast<{CTYPE[it]}>({cv(0, it)} {LOGIC[acc]} {c})"
         (t,) = ot
         ct = CTYPE[t]
+        if op == "add" and t == "u32" and self.mad_adds:
+            return f"op_add_mad({cv(0, t)}, {cv(1, t)}, ctx.cols->one)"
         if op in ARITH:
             return f"static_cast<{ct}>({cv(0, t)} {ARITH[op]} {cv(1, t)})"
         if op in BITS:
@@ -1053,6 +1067,7 @@ def generate(k: Kernel) -> str:
         if heavy:
             body.append("        fresh = false;")
         body.append(f"        if constexpr(kProf) count_block(ctx, {b}, {len(blk.instrs)}u);")
+        L.mad_adds = not headers and bit_heavy(blk)
         body.extend(L.body(blk.instrs, "        ", live_outs[b], b))
         if copies > 1:
             # iterations until the budget has to be looked at again, run in

@@ -48,7 +48,7 @@ struct Columns
     // constant offsets, one instruction a read instead of three.  0: larger,
     // or unknown.
     unsigned                  table_flat;
-    unsigned                  pad0;
+    unsigned                  one; // 1, which the compiler does not know (op_add_mad)
 };
 
 /// An index of such a table plus a record's span (below 64) does not wrap in
@@ -144,6 +144,13 @@ loop_more_ne(const T i, const T n, const unsigned most)
 {
     using U = std::make_unsigned_t<T>;
     return loop_more<U>(static_cast<U>(n) - static_cast<U>(i) - 1u, most);
+}
+
+/// a + b on the multiply-add pipe (`one` is Columns::one).
+__device__ __forceinline__ unsigned
+op_add_mad(const unsigned a, const unsigned b, const unsigned one)
+{
+    return a * one + b;
 }
 
 /// Whether v differs from a 32-bit literal.

@@ -131,9 +131,9 @@ struct K
     L_B0_again:
         fresh = false;
         if constexpr(kProf) count_block(ctx, 0, 282u);
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(((unsigned int)0xdeadull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0xbeefull))));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(((unsigned int)0xdeadull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0xbeefull)), ctx.cols->one));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0xdull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0xdull))));
@@ -141,7 +141,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0xfull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0xfull))));
@@ -149,7 +149,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x1aull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x1aull))));
@@ -157,7 +157,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x6ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x6ull))));
@@ -165,10 +165,10 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(((unsigned int)0xbeefull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x1bd17b98ull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(((unsigned int)0xbeefull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x1bd17b98ull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x1ull)), ctx.cols->one));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x11ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x11ull))));
@@ -176,7 +176,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x1dull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x1dull))));
@@ -184,7 +184,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x10ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x10ull))));
@@ -192,7 +192,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x18ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x18ull))));
@@ -200,10 +200,10 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(((unsigned int)0x1bd17b98ull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0xdeadull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x2ull))));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(((unsigned int)0x1bd17b98ull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0xdeadull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x2ull)), ctx.cols->one));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0xdull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0xdull))));
@@ -211,7 +211,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0xfull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0xfull))));
@@ -219,7 +219,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x1aull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x1aull))));
@@ -227,7 +227,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x6ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x6ull))));
@@ -235,10 +235,10 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(((unsigned int)0xdeadull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0xbeefull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x3ull))));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(((unsigned int)0xdeadull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0xbeefull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x3ull)), ctx.cols->one));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x11ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x11ull))));
@@ -246,7 +246,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x1dull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x1dull))));
@@ -254,7 +254,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x10ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x10ull))));
@@ -262,7 +262,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x18ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x18ull))));
@@ -270,10 +270,10 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(((unsigned int)0xbeefull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x1bd17b98ull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x4ull))));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(((unsigned int)0xbeefull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x1bd17b98ull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x4ull)), ctx.cols->one));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0xdull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0xdull))));
@@ -281,7 +281,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0xfull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0xfull))));
@@ -289,7 +289,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x1aull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x1aull))));
@@ -297,7 +297,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x6ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x6ull))));
@@ -305,10 +305,10 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(((unsigned int)0x1bd17b98ull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0xdeadull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x5ull))));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(((unsigned int)0x1bd17b98ull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0xdeadull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x5ull)), ctx.cols->one));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x11ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x11ull))));
@@ -316,7 +316,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x1dull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x1dull))));
@@ -324,7 +324,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x10ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x10ull))));
@@ -332,7 +332,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x18ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x18ull))));
@@ -340,10 +340,10 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(((unsigned int)0xdeadull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0xbeefull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x6ull))));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(((unsigned int)0xdeadull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0xbeefull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x6ull)), ctx.cols->one));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0xdull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0xdull))));
@@ -351,7 +351,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0xfull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0xfull))));
@@ -359,7 +359,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x1aull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x1aull))));
@@ -367,7 +367,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x6ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x6ull))));
@@ -375,10 +375,10 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(((unsigned int)0xbeefull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x1bd17b98ull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x7ull))));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(((unsigned int)0xbeefull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x1bd17b98ull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x7ull)), ctx.cols->one));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x11ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x11ull))));
@@ -386,7 +386,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x1dull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x1dull))));
@@ -394,7 +394,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x10ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x10ull))));
@@ -402,7 +402,7 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(R.r1)));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(R.r1), ctx.cols->one));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x18ull)) & static_cast<unsigned int>(((unsigned int)0x1full))));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) << static_cast<unsigned int>(R.r2)));
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(((unsigned int)0x20ull)) - static_cast<unsigned int>(((unsigned int)0x18ull))));
@@ -410,9 +410,9 @@ struct K
         R.r3 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) >> static_cast<unsigned int>(R.r3)));
         R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) | static_cast<unsigned int>(R.r3)));
         R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) ^ static_cast<unsigned int>(R.r0)));
-        R.r0 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r0) + static_cast<unsigned int>(((unsigned int)0x1bd17b98ull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0xdeadull))));
-        R.r1 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r1) + static_cast<unsigned int>(((unsigned int)0x8ull))));
+        R.r0 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r0), static_cast<unsigned int>(((unsigned int)0x1bd17b98ull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0xdeadull)), ctx.cols->one));
+        R.r1 = static_cast<unsigned int>(op_add_mad(static_cast<unsigned int>(R.r1), static_cast<unsigned int>(((unsigned int)0x8ull)), ctx.cols->one));
         goto L_HALT;
     L_HALT:
         return kHalt;

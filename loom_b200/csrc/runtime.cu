@@ -558,6 +558,7 @@ launch(loom_b200_handle* h, const loom_b200_launch& L, cudaStream_t stream, uint
     cols.inst_start = reinterpret_cast<const unsigned long long*>(L.instance_starts);
     cols.num_inst   = L.instance_starts ? L.num_instances : 0u;
     cols.table      = L.table;
+    cols.one        = 1u;
     cols.table_flat = table_flat(L.table, L.table_words) ? 1u : 0u;
     cols.tid_base   = first; // thread ids in flight lie in [first, first + n)
     const loom_b200_opts& o = h->opts;

@@ -629,6 +629,7 @@ slice_launch(loom_b200_server* s, unsigned ctas_per_sm)
     c.inst_start = s->d_starts;
     c.num_inst   = static_cast<unsigned>(m);
     c.table      = s->d_table;
+    c.one        = 1u;
     c.table_flat = flat_table(s->cfg) ? 1u : 0u;
     c.ring_mask  = s->mask;
     c.tid_base   = tid_base(s);

@@ -164,6 +164,7 @@ loom_b200_launch_static(const char*             kernel,
     cols.inst_start = reinterpret_cast<const unsigned long long*>(L->instance_starts);
     cols.num_inst   = L->instance_starts ? L->num_instances : 0u;
     cols.table      = L->table;
+    cols.one        = 1u;
     cols.table_flat = table_flat(L->table, L->table_words) ? 1u : 0u;
 
     loom_b200_opts o{};
