@@ -1382,13 +1382,17 @@ def generate(k: Kernel) -> str:
     w(f"const unsigned kRegCaps[] = {{{', '.join(f'{c}u' for c in caps)}}};")
     w("")
     w("/// The megakernel at register cap `regs` (0: the default), in its form")
-    w("/// for launches that never park when `park` is false; profiled launches")
+    w("/// for launches of `form`; profiled launches")
     w("/// and launches with the staged restore (`bulk`) use the default cap and")
     w("/// the parking form, and so do launches of a kernel with table records on")
     w("/// a table that is not flat (the staged-restore instantiation reads")
     w("/// every word by its own index).  NULL: no such cap compiled.")
-    w("const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park, bool flat)")
+    w("const void* regroup_fn(unsigned regs, bool profile, bool bulk, RegroupForm form, bool flat)")
     w("{")
+    ordered = len(k.step_headers(set(long_blocks(k)))) > 1
+    if ordered:
+        w("    const bool ordered = form == RegroupForm::kParkOrdered && (regs == 0u || regs == K::kRegroupMaxRegs) && !bulk && flat;")
+        w("    if(profile && ordered) return reinterpret_cast<const void*>(&regroup_kernel<K, true, K::kRegroupMaxRegs, false, true, true>);")
     w("    if(profile) return reinterpret_cast<const void*>(&regroup_kernel<K, true, K::kRegroupMaxRegs, true>);")
     w("    if(bulk) return reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, true>);")
     w("    if(K::kTableRows && !flat)")
@@ -1397,6 +1401,9 @@ def generate(k: Kernel) -> str:
     w("        for(const unsigned c: kRegCaps) known |= c == regs;")
     w("        return known ? reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, true>) : nullptr;")
     w("    }")
+    w("    const bool park = form != RegroupForm::kNeverPark;")
+    if ordered:
+        w("    if(ordered) return reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, false, true, true>);")
     w("    switch(regs)")
     w("    {")
     w("    case 0u:")
@@ -1410,7 +1417,7 @@ def generate(k: Kernel) -> str:
     w("cudaError_t launch_regroup(const RegroupLaunch& a)")
     w("{")
     w("    void* args[] = {const_cast<RegroupParams*>(&a.params)};")
-    w("    const void* fn = regroup_fn(a.regs, a.profile, a.params.bulk_restore != 0u, a.park, a.params.cols.table_flat != 0u);")
+    w("    const void* fn = regroup_fn(a.regs, a.profile, a.params.bulk_restore != 0u, a.form, a.params.cols.table_flat != 0u);")
     w("    if(!fn) return cudaErrorInvalidValue;")
     w("    if(a.dyn_smem)")
     w("    {")
@@ -1423,10 +1430,10 @@ def generate(k: Kernel) -> str:
     w("    return cudaLaunchCooperativeKernel(fn, dim3(a.grid), dim3(a.block), args, a.dyn_smem, a.stream);")
     w("}")
     w("")
-    w("cudaError_t regroup_occupancy(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park, bool flat,")
+    w("cudaError_t regroup_occupancy(int block, bool profile, unsigned regs, unsigned dyn_smem, RegroupForm form, bool flat,")
     w("                              int* ctas)")
     w("{")
-    w("    const void* fn = regroup_fn(regs, profile, dyn_smem != 0u, park, flat);")
+    w("    const void* fn = regroup_fn(regs, profile, dyn_smem != 0u, form, flat);")
     w("    if(!fn) return cudaErrorInvalidValue;")
     w("    if(dyn_smem)")
     w("    {")

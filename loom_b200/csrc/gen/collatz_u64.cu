@@ -450,12 +450,12 @@ cudaError_t plain_regs(bool profile, bool flat, int* regs)
 const unsigned kRegCaps[] = {64u, 40u, 48u};
 
 /// The megakernel at register cap `regs` (0: the default), in its form
-/// for launches that never park when `park` is false; profiled launches
+/// for launches of `form`; profiled launches
 /// and launches with the staged restore (`bulk`) use the default cap and
 /// the parking form, and so do launches of a kernel with table records on
 /// a table that is not flat (the staged-restore instantiation reads
 /// every word by its own index).  NULL: no such cap compiled.
-const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park, bool flat)
+const void* regroup_fn(unsigned regs, bool profile, bool bulk, RegroupForm form, bool flat)
 {
     if(profile) return reinterpret_cast<const void*>(&regroup_kernel<K, true, K::kRegroupMaxRegs, true>);
     if(bulk) return reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, true>);
@@ -465,6 +465,7 @@ const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park, bool f
         for(const unsigned c: kRegCaps) known |= c == regs;
         return known ? reinterpret_cast<const void*>(&regroup_kernel<K, false, K::kRegroupMaxRegs, true>) : nullptr;
     }
+    const bool park = form != RegroupForm::kNeverPark;
     switch(regs)
     {
     case 0u:
@@ -481,7 +482,7 @@ const void* regroup_fn(unsigned regs, bool profile, bool bulk, bool park, bool f
 cudaError_t launch_regroup(const RegroupLaunch& a)
 {
     void* args[] = {const_cast<RegroupParams*>(&a.params)};
-    const void* fn = regroup_fn(a.regs, a.profile, a.params.bulk_restore != 0u, a.park, a.params.cols.table_flat != 0u);
+    const void* fn = regroup_fn(a.regs, a.profile, a.params.bulk_restore != 0u, a.form, a.params.cols.table_flat != 0u);
     if(!fn) return cudaErrorInvalidValue;
     if(a.dyn_smem)
     {
@@ -494,10 +495,10 @@ cudaError_t launch_regroup(const RegroupLaunch& a)
     return cudaLaunchCooperativeKernel(fn, dim3(a.grid), dim3(a.block), args, a.dyn_smem, a.stream);
 }
 
-cudaError_t regroup_occupancy(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park, bool flat,
+cudaError_t regroup_occupancy(int block, bool profile, unsigned regs, unsigned dyn_smem, RegroupForm form, bool flat,
                               int* ctas)
 {
-    const void* fn = regroup_fn(regs, profile, dyn_smem != 0u, park, flat);
+    const void* fn = regroup_fn(regs, profile, dyn_smem != 0u, form, flat);
     if(!fn) return cudaErrorInvalidValue;
     if(dyn_smem)
     {

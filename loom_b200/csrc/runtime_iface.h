@@ -24,6 +24,33 @@ struct PlainLaunch
     cudaStream_t        stream;
 };
 
+/// Instantiations of the megakernel.
+enum class RegroupForm : unsigned
+{
+    kNeverPark,   // schedule 2 or 3, no period, no prefetch: no queue code
+    kPark,        // every other launch but those of kParkOrdered
+    kParkOrdered, // schedules 0 and 1 without the cost model: bursts in MinPC
+                  // order (programs of several loops, the default register cap)
+};
+
+/// The form that a launch with these options runs.
+inline RegroupForm
+regroup_form(const loom_b200_opts& o)
+{
+    const bool never = (o.schedule == 2u || o.schedule == 3u) && o.period == LOOM_B200_PERIOD_UNBOUNDED;
+    if(never && o.no_prefetch) return RegroupForm::kNeverPark;
+    return o.schedule < 2u && !o.cost_model ? RegroupForm::kParkOrdered : RegroupForm::kPark;
+}
+
+/// ... where its threads may have to wait for another launch in the queues (a
+/// server's slices), or the queues are there anyway.
+inline RegroupForm
+parking_form(const loom_b200_opts& o)
+{
+    const RegroupForm f = regroup_form(o);
+    return f == RegroupForm::kNeverPark ? RegroupForm::kPark : f;
+}
+
 struct RegroupLaunch
 {
     RegroupParams params;
@@ -37,9 +64,7 @@ struct RegroupLaunch
     // resident together, as the grid barrier between rounds needs)
     bool          ordinary = false;
     unsigned      dyn_smem = 0; // dynamic shared memory (bulk_restore's staging)
-    // false: the launch never parks (schedule 2 or 3, no period), does not
-    // prefetch and runs the megakernel compiled without queue code
-    bool          park = true;
+    RegroupForm   form = RegroupForm::kPark;
     cudaStream_t  stream;
 };
 
@@ -67,7 +92,7 @@ struct KernelEntry
     unsigned                     num_queues; // work queues of the regrouping engine
     cudaError_t (*plain)(const PlainLaunch&);
     cudaError_t (*regroup)(const RegroupLaunch&);
-    cudaError_t (*regroup_occupancy)(int block, bool profile, unsigned regs, unsigned dyn_smem, bool park,
+    cudaError_t (*regroup_occupancy)(int block, bool profile, unsigned regs, unsigned dyn_smem, RegroupForm form,
                                      bool flat, int* ctas_per_sm);
     cudaError_t (*plain_regs)(bool profile, bool flat, int* regs); // registers per thread of the plain kernel
     const loom_b200_queue_layout* queues;   // num_queues entries

@@ -457,7 +457,7 @@ loom_b200_server_create(const char*                 kernel,
     int      ctas  = 0;
     for(;;)
     {
-        if(e->regroup_occupancy(static_cast<int>(block), o.profile != 0, o.max_regs, 0u, true,
+        if(e->regroup_occupancy(static_cast<int>(block), o.profile != 0, o.max_regs, 0u, parking_form(o),
                                 flat_table(*cfg), &ctas) != cudaSuccess)
         {
             delete s;
@@ -668,13 +668,14 @@ slice_launch(loom_b200_server* s, unsigned ctas_per_sm)
         // never more CTAs per SM than fit (cooperative launches need every
         // CTA resident at once)
         int fit = 0;
-        SV_CUDA(s->e->regroup_occupancy(static_cast<int>(s->block), o.profile != 0, o.max_regs, 0u, true,
+        SV_CUDA(s->e->regroup_occupancy(static_cast<int>(s->block), o.profile != 0, o.max_regs, 0u, parking_form(o),
                                         flat_table(s->cfg), &fit));
         const unsigned c = std::min<unsigned>(ctas_per_sm, static_cast<unsigned>(std::max(fit, 1)));
         L.grid           = c * static_cast<unsigned>(s->sms);
     }
     L.block   = s->block;
     L.regs    = o.max_regs;
+    L.form    = parking_form(o);
     L.profile = o.profile != 0;
     L.stream  = s->stream;
     SV_CUDA(cudaEventRecord(s->ev_a, s->stream));

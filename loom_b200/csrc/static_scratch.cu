@@ -205,7 +205,8 @@ loom_b200_launch_static(const char*             kernel,
     int      ctas  = 0;
     for(;;)
     {
-        if(e->regroup_occupancy(static_cast<int>(block), false, 0u, 0u, true, cols.table_flat != 0u, &ctas) != cudaSuccess)
+        if(e->regroup_occupancy(static_cast<int>(block), false, 0u, 0u, parking_form(o), cols.table_flat != 0u,
+                                &ctas) != cudaSuccess)
             return LOOM_B200_ERR_CUDA;
         if(ctas > 0 || block <= 32) break;
         block /= 2;
@@ -237,6 +238,7 @@ loom_b200_launch_static(const char*             kernel,
     R.params.schedule      = o.schedule;
     R.grid                 = static_cast<unsigned>(ctas * slot.sms);
     R.block                = block;
+    R.form                 = parking_form(o);
     R.profile              = false;
     R.stream               = static_cast<cudaStream_t>(stream_);
 
