@@ -883,6 +883,7 @@ def generate(k: Kernel) -> str:
     w(f"    static constexpr int kRegroupMaxRegs = {REGROUP_MAX_REGS};")
     # small kernels: two inlined copies of their code in the megakernel
     w(f"    static constexpr bool kSplitCallSites = {'true' if sum(counts) <= REG_VARIANT_MIN_INSTR else 'false'};")
+    w(f"    static constexpr int kStepHeaders = {len(k.step_headers(set(long_blocks(k))))}; // blocks where a step may end")
     # kernels that read records of the table: their launches on flat tables
     # run instantiations of their own
     table_rows = any(L.table_rows(b.instrs)[0] for b in k.blocks)

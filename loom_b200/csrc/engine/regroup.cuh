@@ -459,6 +459,16 @@ regroup_kernel(const RegroupParams p)
                         run = rk == lo;
                         if(run) --visits;
                     }
+                    else if(minpc && K::kStepHeaders <= 1)
+                    {
+                        // one loop: no order to keep, so no ranks to read
+                        // and no minimum to vote (Collatz, 2^24 threads 2.29
+                        // -> 2.03 ms; with two loops a ballot per block where
+                        // lanes can stand was slower than the vote, 22.8 ->
+                        // 23.2 ms on the 1024x768x64 render)
+                        run = pc >= 0;
+                        if(__ballot_sync(FULL, run) == 0u) break;
+                    }
                     else if(minpc)
                     {
                         unsigned rk = pc >= 0 ? s_rank[pc] : 0xffffffffu;

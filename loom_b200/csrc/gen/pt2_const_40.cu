@@ -22,6 +22,7 @@ struct K
     static constexpr int kNumQueues = 55;
     static constexpr int kRegroupMaxRegs = 64;
     static constexpr bool kSplitCallSites = false;
+    static constexpr int kStepHeaders = 5; // blocks where a step may end
     static constexpr bool kTableRows = false;
     struct Regs
     {
