@@ -1360,13 +1360,14 @@ def generate(k: Kernel) -> str:
     w("cudaError_t launch_plain(const PlainLaunch& a)")
     w("{")
     w("    const bool               flat = a.cols.table_flat != 0u;")
-    w("    const unsigned long long cta  = static_cast<unsigned long long>(a.block) * a.per;")
+    w("    const unsigned long long cta  = a.lanes < 32u ? a.lanes : static_cast<unsigned long long>(a.block) * a.per;")
     w("    const unsigned long long grid = (a.n + cta - 1) / cta;")
     w("    if(grid == 0) return cudaSuccess;")
     w("    const void* fn     = plain_fn(a.profile, flat, a.per);")
     w("    void*       args[] = {const_cast<Columns*>(&a.cols), const_cast<unsigned long long*>(&a.first),")
     w("                          const_cast<unsigned long long*>(&a.n), const_cast<unsigned long long*>(&a.max_steps),")
-    w("                          const_cast<unsigned**>(&a.status), const_cast<unsigned long long**>(&a.counters)};")
+    w("                          const_cast<unsigned**>(&a.status), const_cast<unsigned long long**>(&a.counters),")
+    w("                          const_cast<unsigned*>(&a.lanes)};")
     w("    return cudaLaunchKernel(fn, dim3(static_cast<unsigned>(grid)), dim3(a.block), args, 0, a.stream);")
     w("}")
     w("")

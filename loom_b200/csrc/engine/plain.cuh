@@ -23,7 +23,8 @@ constexpr unsigned kStraightPer = 4;
 /// once, registers live in CUDA registers; counters[0..1] receive
 /// thread/warp VM-instruction totals when kProf is set (lane efficiency =
 /// counters[0] / (32 * counters[1])).  kFlat: the launch's table is flat
-/// (only kernels that read table records have that instantiation).
+/// (only kernels that read table records have that instantiation).  With
+/// lanes < 32 (CTAs of one warp) a warp runs that many Loom threads.
 template <typename K, bool kProf, bool kFlat, unsigned kPer>
 __global__ void
 plain_kernel(const Columns                  cols,
@@ -31,12 +32,16 @@ plain_kernel(const Columns                  cols,
              const unsigned long long       n,
              const unsigned long long       max_steps,
              unsigned* __restrict__         status,
-             unsigned long long* __restrict__ counters)
+             unsigned long long* __restrict__ counters,
+             const unsigned                 lanes)
 {
     __shared__ unsigned long long s_blk[2 * (kProf ? K::kNumBlocks : 1)];
     Ctx ctx{0ull, 0ull, status, &cols, kProf ? s_blk : nullptr};
     if constexpr(kProf) block_counters_clear(s_blk, K::kNumBlocks);
-    const unsigned long long i0 = static_cast<unsigned long long>(blockIdx.x) * blockDim.x * kPer + threadIdx.x;
+    // lanes < 32 (small launches, CTAs of one warp): only the first lanes of
+    // a warp hold threads
+    const unsigned long long i0 = static_cast<unsigned long long>(blockIdx.x) * (lanes < 32u ? lanes : blockDim.x * kPer) +
+                                  (threadIdx.x < lanes || lanes == 32u ? threadIdx.x : n);
     // the block budget is the step guard: a thread that has not halted
     // when it runs out is stopped and flagged
     const unsigned budget = max_steps < 0xffffffffull

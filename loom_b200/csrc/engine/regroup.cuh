@@ -284,6 +284,16 @@ regroup_kernel(const RegroupParams p)
     typename K::In     pf;
     unsigned long long pf_tid = ~0ull;
     const bool         cost_on = p.cost_model != 0u;
+    // A launch of fewer threads than the grid has lanes: each warp takes its
+    // share of them only (and prefetches none), as a warp takes as long as
+    // the paths of all its threads together: 8192 threads of the sphere path
+    // tracer 177 -> 119 us at its tuned options.  Schedules 0 and 1 keep whole
+    // warps: a group under its quorum would park.
+    const unsigned long long all_warps = static_cast<unsigned long long>(gridDim.x) * (blockDim.x >> 5);
+    const unsigned long long all_n     = p.n - p.cols.tid_base;
+    const unsigned           share     = p.schedule >= 2u && p.slice_rounds == 0u && all_n < 32ull * all_warps
+                                             ? static_cast<unsigned>((all_n + all_warps - 1) / all_warps) : 32u;
+    const unsigned           first_claim = share < 32u ? (1u << share) - 1u : FULL;
     // staged restore: this warp's mbarrier and staging area
     extern __shared__ __align__(16) unsigned char s_dyn[];
     const unsigned      wib   = threadIdx.x >> 5;
@@ -408,7 +418,7 @@ regroup_kernel(const RegroupParams p)
             else
             {
                 if(dry) break;
-                const unsigned long long t = claim_inputs(FULL, p.ctl, admit_end, dry);
+                const unsigned long long t = claim_inputs(first_claim, p.ctl, admit_end, dry);
                 if(__ballot_sync(FULL, t != ~0ull) == 0u) break;
                 if(t != ~0ull) { typename K::In in; K::load_in(in, p.cols, t); K::start(R, in); tid = t; pc = 0; }
                 tb = 0; tk = 32u;
@@ -418,7 +428,7 @@ regroup_kernel(const RegroupParams p)
             unsigned steps = 0;
             for(;;)
             {
-                if(kPark && p.prefetch && !dry)
+                if(kPark && p.prefetch && !dry && share == 32u)
                 {
                     const unsigned need = __ballot_sync(FULL, pf_tid == ~0ull);
                     if(need)

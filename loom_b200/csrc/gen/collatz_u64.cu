@@ -429,13 +429,14 @@ const void* plain_fn(bool profile, bool flat, unsigned per)
 cudaError_t launch_plain(const PlainLaunch& a)
 {
     const bool               flat = a.cols.table_flat != 0u;
-    const unsigned long long cta  = static_cast<unsigned long long>(a.block) * a.per;
+    const unsigned long long cta  = a.lanes < 32u ? a.lanes : static_cast<unsigned long long>(a.block) * a.per;
     const unsigned long long grid = (a.n + cta - 1) / cta;
     if(grid == 0) return cudaSuccess;
     const void* fn     = plain_fn(a.profile, flat, a.per);
     void*       args[] = {const_cast<Columns*>(&a.cols), const_cast<unsigned long long*>(&a.first),
                           const_cast<unsigned long long*>(&a.n), const_cast<unsigned long long*>(&a.max_steps),
-                          const_cast<unsigned**>(&a.status), const_cast<unsigned long long**>(&a.counters)};
+                          const_cast<unsigned**>(&a.status), const_cast<unsigned long long**>(&a.counters),
+                          const_cast<unsigned*>(&a.lanes)};
     return cudaLaunchKernel(fn, dim3(static_cast<unsigned>(grid)), dim3(a.block), args, 0, a.stream);
 }
 

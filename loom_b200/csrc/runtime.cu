@@ -245,6 +245,14 @@ constexpr unsigned           kDefaultRegroupBlock = 256;
 // per CUDA thread: where the GPU is still full of CUDA threads.  2e7 Threefry
 // counters 147 -> 130 us with 4 (2 and 8 a few per cent slower).
 constexpr unsigned long long kStraightFill        = 2048ull * kStraightPer;
+// Warps per SM that a small launch of a large kernel with loops is spread over:
+// a warp takes as long as the paths of all its threads together, so where
+// warps are to spare it holds fewer of them (sphere path tracer, one per CUDA
+// thread: 768 threads 356 -> 61 us, 8192 threads 312 -> 113 us, 24576 threads
+// 336 -> 223 us; 4, 8 and 24 warps per SM: 138, 156 and 112 us at 8192, and
+// Loom's pt_const at 10000 pixels 25.2, 25.9, 26.3 and 30.1 ms with 4, 8, 16
+// and 24).
+constexpr unsigned           kSpreadWarps         = 16;
 constexpr int                kOneWarpRegs         = 57; // allocated in steps of 8: 65536 / (64 * 32) = 32 warps
 constexpr unsigned           kDefaultUtr         = 16;
 constexpr unsigned           kDefaultPeriod      = 1024;
@@ -498,6 +506,11 @@ plain_block(loom_b200_handle* h, PlainLaunch& L)
         blk = regs >= kOneWarpRegs ? 32u : kDefaultPlainBlock;
     }
     L.block = blk;
+    if(blk == 32u && h->e->per == 1u)
+    {
+        const unsigned long long warps = static_cast<unsigned long long>(h->sms) * kSpreadWarps;
+        while(L.lanes > 1u && L.n <= L.lanes / 2u * warps) L.lanes /= 2u;
+    }
     return LOOM_B200_OK;
 }
 
@@ -657,6 +670,7 @@ launch(loom_b200_handle* h, const loom_b200_launch& L, cudaStream_t stream, uint
         L.block     = o.block_size;
         L.profile   = o.profile != 0;
         L.per       = n >= kStraightFill * h->sms && o.profile == 0 ? e.per : 1u;
+        L.lanes     = 32u;
         L.stream    = stream;
         if(h->own_block)
         {
@@ -664,7 +678,7 @@ launch(loom_b200_handle* h, const loom_b200_launch& L, cudaStream_t stream, uint
             if(rc) return rc;
         }
         LB_CUDA(e.plain(L));
-        const uint64_t cta = static_cast<uint64_t>(L.block) * L.per;
+        const uint64_t cta = L.lanes < 32u ? L.lanes : static_cast<uint64_t>(L.block) * L.per;
         h->last_grid       = static_cast<unsigned>((n + cta - 1) / cta);
         h->plain_threads += n;
     }

@@ -20,6 +20,7 @@ struct PlainLaunch
     unsigned long long* counters;
     unsigned            block;
     bool                profile;
+    unsigned            lanes; // threads per warp (below 32: CTAs of one warp)
     unsigned            per; // Loom threads per CUDA thread: 1, or KernelEntry::per
     cudaStream_t        stream;
 };
