@@ -454,10 +454,13 @@ SCT_MIN = 3
 
 
 class Lowering:
-    def __init__(self, k: Kernel):
+    def __init__(self, k: Kernel, device: bool = False):
         self.k = k
         self.pc = k.pc_reg()
         self.regs = {r.idx: r for r in k.regs}
+        # expressions for device code (the CPU restatement of the gang engine
+        # lowers with this class too, without the device's helpers)
+        self.device = device
         self.mad_adds = False
 
     # ------------------------------------------------------------ views
@@ -529,7 +532,7 @@ class Lowering:
             return f"static_cast<{ct}>({cv(0, t)} {ARITH[op]} {cv(1, t)})"
         if op in BITS:
             return f"static_cast<{ct}>({cv(0, t)} {BITS[op]} {cv(1, t)})"
-        if op in ("eq", "ne") and t in ("u64", "i64"):
+        if op in ("eq", "ne") and t in ("u64", "i64") and self.device:
             # against a literal below 2^32: one three-input logic operation
             # on the halves that sets the predicate, instead of a compare of
             # each half (the ALU pipe takes two cycles for either)
@@ -819,7 +822,7 @@ def pack_slots(items, start: int) -> Dict:
 
 
 def generate(k: Kernel) -> str:
-    L = Lowering(k)
+    L = Lowering(k, device=True)
     name = k.name
     nb = k.num_blocks
     nin = len(k.inputs)
