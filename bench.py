@@ -48,6 +48,7 @@ seeded sample of threads are compared bit for bit with both engines'.
 from __future__ import annotations
 
 import argparse
+import concurrent.futures
 import json
 import math
 import os
@@ -516,8 +517,10 @@ def _cpu_model() -> str:
 
 
 def _reference_runner():
-    """Loom's bse (oracle/_ref) on all host cores, else the C restatement on
-    one core: returns (run(kernel, inputs, table) -> outputs, kind, cores)."""
+    """Loom's bse (oracle/_ref) on all host cores, else the C restatement,
+    slices of the threads on all host cores too (the C call releases the
+    interpreter lock): returns (run(kernel, inputs, table) -> outputs, kind,
+    cores)."""
     from oracle import oracle as O
 
     cores = os.cpu_count() or 1
@@ -529,9 +532,18 @@ def _reference_runner():
         return run, "reference", cores
 
     def run(kernel, ins, table):
-        return O.Interp(kernel).run(ins, table=table)
+        n = len(next(a for a in ins if a is not None))
+        cut = np.linspace(0, n, min(n, 4 * cores) + 1).astype(np.int64)
 
-    return run, "port", 1
+        def part(k):
+            a, b = int(cut[k]), int(cut[k + 1])
+            return O.Interp(kernel).run([None if x is None else x[a:b] for x in ins], n=b - a, table=table)
+
+        with concurrent.futures.ThreadPoolExecutor(cores) as ex:
+            parts = list(ex.map(part, range(len(cut) - 1)))
+        return [np.concatenate(c) for c in zip(*parts)]
+
+    return run, "port", cores
 
 
 def cpu_reference(w, check_tids=None, target_s: float = 2.0):
@@ -559,7 +571,7 @@ def cpu_reference(w, check_tids=None, target_s: float = 2.0):
     how = (
         "Loom bse (vm::bse::function), g++ -O3 -march=x86-64-v4 -mfma -ffp-contract=off, one std::thread per core"
         if kind == "reference"
-        else "C restatement of bse, one thread"
+        else "C restatement of bse, one thread per core"
     )
     info = {
         "unit": "Msamples/s",
