@@ -887,6 +887,8 @@ def generate(k: Kernel) -> str:
     # small kernels: two inlined copies of their code in the megakernel
     w(f"    static constexpr bool kSplitCallSites = {'true' if sum(counts) <= REG_VARIANT_MIN_INSTR else 'false'};")
     w(f"    static constexpr int kStepHeaders = {len(k.step_headers(set(long_blocks(k))))}; // blocks where a step may end")
+    spread = bool(k.loop_headers()) and sum(counts) > REG_VARIANT_MIN_INSTR
+    w(f"    static constexpr bool kSpread = {str(spread).lower()}; // a large program with loops")
     # kernels that read records of the table: their launches on flat tables
     # run instantiations of their own
     table_rows = any(L.table_rows(b.instrs)[0] for b in k.blocks)
@@ -1458,7 +1460,7 @@ def generate(k: Kernel) -> str:
     w(f"    &loom_b200::k_{name}::regroup_occupancy,")
     w(f"    &loom_b200::k_{name}::plain_regs,")
     w(f"    loom_b200::k_{name}::kQueues, loom_b200::k_{name}::kSegments,")
-    w(f"    loom_b200::k_{name}::kRegCaps, {len(caps)}u, loom_b200::k_{name}::K::kMaxStageRow, {"loom_b200::kStraightPer" if several else "1u"}}};")
+    w(f"    loom_b200::k_{name}::kRegCaps, {len(caps)}u, loom_b200::k_{name}::K::kMaxStageRow, loom_b200::k_{name}::K::kSpread, {"loom_b200::kStraightPer" if several else "1u"}}};")
     return "\n".join(o) + "\n"
 
 

@@ -38,10 +38,12 @@ plain_kernel(const Columns                  cols,
     __shared__ unsigned long long s_blk[2 * (kProf ? K::kNumBlocks : 1)];
     Ctx ctx{0ull, 0ull, status, &cols, kProf ? s_blk : nullptr};
     if constexpr(kProf) block_counters_clear(s_blk, K::kNumBlocks);
-    // lanes < 32 (small launches, CTAs of one warp): only the first lanes of
+    // lanes < 32 (small launches of large kernels, CTAs of one warp): only the first lanes of
     // a warp hold threads
-    const unsigned long long i0 = static_cast<unsigned long long>(blockIdx.x) * (lanes < 32u ? lanes : blockDim.x * kPer) +
-                                  (threadIdx.x < lanes || lanes == 32u ? threadIdx.x : n);
+    const unsigned long long i0 =
+        K::kSpread && lanes < 32u
+            ? static_cast<unsigned long long>(blockIdx.x) * lanes + (threadIdx.x < lanes ? threadIdx.x : n)
+            : static_cast<unsigned long long>(blockIdx.x) * blockDim.x * kPer + threadIdx.x;
     // the block budget is the step guard: a thread that has not halted
     // when it runs out is stopped and flagged
     const unsigned budget = max_steps < 0xffffffffull

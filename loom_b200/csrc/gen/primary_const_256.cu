@@ -23,6 +23,7 @@ struct K
     static constexpr int kRegroupMaxRegs = 64;
     static constexpr bool kSplitCallSites = false;
     static constexpr int kStepHeaders = 5; // blocks where a step may end
+    static constexpr bool kSpread = true; // a large program with loops
     static constexpr bool kTableRows = false;
     struct Regs
     {
@@ -6042,4 +6043,4 @@ const loom_b200::KernelEntry loom_b200_entry_primary_const_256 = {
     &loom_b200::k_primary_const_256::regroup_occupancy,
     &loom_b200::k_primary_const_256::plain_regs,
     loom_b200::k_primary_const_256::kQueues, loom_b200::k_primary_const_256::kSegments,
-    loom_b200::k_primary_const_256::kRegCaps, 8u, loom_b200::k_primary_const_256::K::kMaxStageRow, 1u};
+    loom_b200::k_primary_const_256::kRegCaps, 8u, loom_b200::k_primary_const_256::K::kMaxStageRow, loom_b200::k_primary_const_256::K::kSpread, 1u};

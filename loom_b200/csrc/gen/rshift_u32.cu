@@ -19,6 +19,7 @@ struct K
     static constexpr int kRegroupMaxRegs = 64;
     static constexpr bool kSplitCallSites = true;
     static constexpr int kStepHeaders = 0; // blocks where a step may end
+    static constexpr bool kSpread = false; // a large program with loops
     static constexpr bool kTableRows = false;
     struct Regs
     {
@@ -343,4 +344,4 @@ const loom_b200::KernelEntry loom_b200_entry_rshift_u32 = {
     &loom_b200::k_rshift_u32::regroup_occupancy,
     &loom_b200::k_rshift_u32::plain_regs,
     loom_b200::k_rshift_u32::kQueues, loom_b200::k_rshift_u32::kSegments,
-    loom_b200::k_rshift_u32::kRegCaps, 3u, loom_b200::k_rshift_u32::K::kMaxStageRow, loom_b200::kStraightPer};
+    loom_b200::k_rshift_u32::kRegCaps, 3u, loom_b200::k_rshift_u32::K::kMaxStageRow, loom_b200::k_rshift_u32::K::kSpread, loom_b200::kStraightPer};

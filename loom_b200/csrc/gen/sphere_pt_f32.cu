@@ -19,6 +19,7 @@ struct K
     static constexpr int kRegroupMaxRegs = 64;
     static constexpr bool kSplitCallSites = false;
     static constexpr int kStepHeaders = 2; // blocks where a step may end
+    static constexpr bool kSpread = true; // a large program with loops
     static constexpr bool kTableRows = true;
     struct Regs
     {
@@ -5658,4 +5659,4 @@ const loom_b200::KernelEntry loom_b200_entry_sphere_pt_f32 = {
     &loom_b200::k_sphere_pt_f32::regroup_occupancy,
     &loom_b200::k_sphere_pt_f32::plain_regs,
     loom_b200::k_sphere_pt_f32::kQueues, loom_b200::k_sphere_pt_f32::kSegments,
-    loom_b200::k_sphere_pt_f32::kRegCaps, 8u, loom_b200::k_sphere_pt_f32::K::kMaxStageRow, 1u};
+    loom_b200::k_sphere_pt_f32::kRegCaps, 8u, loom_b200::k_sphere_pt_f32::K::kMaxStageRow, loom_b200::k_sphere_pt_f32::K::kSpread, 1u};

@@ -506,7 +506,7 @@ plain_block(loom_b200_handle* h, PlainLaunch& L)
         blk = regs >= kOneWarpRegs ? 32u : kDefaultPlainBlock;
     }
     L.block = blk;
-    if(blk == 32u && h->e->per == 1u)
+    if(blk == 32u && h->e->spread)
     {
         const unsigned long long warps = static_cast<unsigned long long>(h->sms) * kSpreadWarps;
         while(L.lanes > 1u && L.n <= L.lanes / 2u * warps) L.lanes /= 2u;

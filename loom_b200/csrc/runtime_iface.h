@@ -101,6 +101,7 @@ struct KernelEntry
     const unsigned*               reg_caps; // compiled register caps, default first
     unsigned                      num_reg_caps;
     unsigned                      max_stage_row; // K::kMaxStageRow (bulk_restore staging per entry)
+    bool                          spread;        // K::kSpread: small plain launches may use part of a warp's lanes
     unsigned                      per;           // Loom threads per CUDA thread of a large plain launch
 };
 
