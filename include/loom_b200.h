@@ -89,7 +89,9 @@ typedef struct loom_b200_kernel_info
 typedef struct loom_b200_opts
 {
     uint32_t mode;        /* LOOM_B200_PLAIN or LOOM_B200_REGROUP */
-    uint32_t block_size;  /* CUDA threads per CTA (multiple of 32) */
+    uint32_t block_size;  /* CUDA threads per CTA (multiple of 32; 0: 256, and
+                             for plain launches the engine's own choice, one
+                             warp for kernels of many registers) */
     uint32_t utr_lanes;   /* regroup: keep running in registers while the
                              largest same-PC group has >= utr_lanes lanes
                              (the GPU form of Loom's UTR, simd.hpp:3273-3292) */
@@ -221,7 +223,8 @@ typedef struct loom_b200_launch
     uint32_t               num_instances;
     uint32_t               pad;
     const uint32_t*        table;           /* or NULL */
-    uint64_t               table_words;
+    uint64_t               table_words;     /* device launches: 0 = unstated (the
+                                               allocation then bounds it) */
 } loom_b200_launch;
 
 typedef struct loom_b200_handle loom_b200_handle;
