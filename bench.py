@@ -534,10 +534,11 @@ def _reference_runner():
     def run(kernel, ins, table):
         n = len(next(a for a in ins if a is not None))
         cut = np.linspace(0, n, min(n, 4 * cores) + 1).astype(np.int64)
+        interp = O.Interp(kernel)  # parsed once; a run only reads it
 
         def part(k):
             a, b = int(cut[k]), int(cut[k + 1])
-            return O.Interp(kernel).run([None if x is None else x[a:b] for x in ins], n=b - a, table=table)
+            return interp.run([None if x is None else x[a:b] for x in ins], n=b - a, table=table)
 
         with concurrent.futures.ThreadPoolExecutor(cores) as ex:
             parts = list(ex.map(part, range(len(cut) - 1)))

@@ -178,7 +178,8 @@ typedef struct
     block*   blocks;
 } kernel;
 
-static char g_err[256];
+/* the last failed load's message, of the thread that made it */
+static _Thread_local char g_err[256];
 
 const char*
 li_error(void)
@@ -236,8 +237,9 @@ void li_free(void* p);
 static int
 split(char* line, char** tok, int max)
 {
-    int n = 0;
-    for(char* s = strtok(line, " \t\r\n"); s && n < max; s = strtok(NULL, " \t\r\n"))
+    int   n  = 0;
+    char* sv = NULL;
+    for(char* s = strtok_r(line, " \t\r\n", &sv); s && n < max; s = strtok_r(NULL, " \t\r\n", &sv))
         tok[n++] = s;
     return n;
 }
