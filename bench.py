@@ -538,7 +538,9 @@ def _reference_runner():
 
         def part(k):
             a, b = int(cut[k]), int(cut[k + 1])
-            return interp.run([None if x is None else x[a:b] for x in ins], n=b - a, table=table)
+            # a column that is left out is the thread index, which goes on from slice to slice
+            cols = [np.arange(a, b).astype(O.NP_TYPE[t]) if x is None else x[a:b] for x, (_, t) in zip(ins, interp.inputs)]
+            return interp.run(cols, n=b - a, table=table)
 
         with concurrent.futures.ThreadPoolExecutor(cores) as ex:
             parts = list(ex.map(part, range(len(cut) - 1)))

@@ -61,3 +61,22 @@ def test_slices_of_the_cpu_leg_equal_one_run():
             assert len(got) == len(want) and all(g.tobytes() == w.tobytes() for g, w in zip(got, want))
         """
     )
+
+
+def test_slices_continue_the_thread_index():
+    """A column that is left out holds the thread index."""
+    _child(
+        """
+        import numpy as np
+        import bench
+        from oracle import oracle as O
+
+        O.ref_available = lambda: False
+        run, _, _ = bench._reference_runner()
+        for name in ("bit_xor_u16", "bit_or_u64", "minmax_f32"):
+            x = np.arange(300, 0, -1).astype(O.NP_TYPE[O.Interp(name).inputs[0][1]])
+            got = run(name, [x, None], None)
+            want = O.Interp(name).run([x, None], n=len(x))
+            assert all(g.tobytes() == w.tobytes() for g, w in zip(got, want)), name
+        """
+    )
