@@ -354,7 +354,7 @@ def select_arms(instrs, live_out, storage) -> Dict[int, tuple]:
     return out
 
 
-def guarded_region(instrs, live_out, fixed):
+def guarded_region(instrs, live_out, fixed, arms=None):
     """Work of a block that only matters while a condition register holds
     true: (position of the instruction that sets the register, positions of
     the work), or None.
@@ -366,19 +366,34 @@ def guarded_region(instrs, live_out, fixed):
     what else feeds only those has no effect, so a lane whose condition is
     false may skip all of it.  The rest of the block (`fixed` positions are
     part of it, as are instructions with side effects) runs after the region,
-    and only where that order gives the same values.  Of all conditions the
-    one with the costliest region is taken."""
+    and only where that order gives the same values: order meaning that of the
+    generated code, where the arms of a select (`arms`, from select_arms) stand
+    right before it.  Of all conditions the one with the costliest region is
+    taken."""
     best, best_cost = None, SINK_MIN_COST - 1
     n = len(instrs)
     last = n - 1 if n and not isinstance(instrs[-1], Compute) else n
-    for c in range(last):
+    arms = arms or {}
+    moved = {p for line, asm, _ in arms.values() for p in line + asm}
+    # predicated: their results never reach their registers
+    unwritten = {p for _, asm, _ in arms.values() for p in asm}
+    order = []
+    for p in range(last):
+        if p in arms:
+            order += arms[p][0] + arms[p][1]
+        if p not in moved:
+            order.append(p)
+    for at, c in enumerate(order):
         h = instrs[c]
+        if c in moved:
+            continue
+        after = order[at + 1 :]
         if h.op not in CMP and h.op not in LOGIC and h.op != "pacc":
             continue
         reg = h.dst.reg
         known = {reg}  # registers that hold false while the condition does
         noop = set()
-        for q in range(c + 1, last):
+        for q in after:
             ins = instrs[q]
             first = None if not ins.args or ins.args[0].is_literal else ins.args[0].reg
             same = first == ins.dst.reg
@@ -396,19 +411,20 @@ def guarded_region(instrs, live_out, fixed):
         # backwards: what is read while the condition is false
         live = set(live_out) | ({r for r in instrs[-1].reads()} if last < n else set())
         skip = set()
-        for q in range(last - 1, c, -1):
+        for q in reversed(after):
             ins = instrs[q]
             if q in noop and q not in fixed:
                 skip.add(q)
             elif ins.dst.reg in live or q in fixed or ins.op == "assert_fp":
-                live.discard(ins.dst.reg)
+                if q not in unwritten:
+                    live.discard(ins.dst.reg)
                 live |= set(ins.reads())
             else:
                 skip.add(q)
         # the region in order, then the rest: cut where the order matters
         inside = []
         rest = []
-        for q in range(c + 1, last):
+        for q in after:
             ins = instrs[q]
             if q not in skip:
                 rest.append(q)
@@ -427,14 +443,15 @@ def guarded_region(instrs, live_out, fixed):
         if len(inside) != len(skip):
             live = set(live_out) | ({r for r in instrs[-1].reads()} if last < n else set())
             ok = True
-            for q in range(last - 1, c, -1):
+            for q in reversed(after):
                 ins = instrs[q]
                 if q in inside:
                     if q not in noop and ins.dst.reg in live:
                         ok = False
                         break
                     continue
-                live.discard(ins.dst.reg)
+                if q not in unwritten:
+                    live.discard(ins.dst.reg)
                 live |= set(ins.reads())
             if not ok:
                 continue
@@ -715,7 +732,7 @@ class Lowering:
         for pos in rows:
             out.append(inner + f"unsigned {', '.join(f'tw{pos}_{d}' for d in rows[pos][1])};")
         fixed = set(rows) | set(member) | set(sct_of) | set(arms) | in_arm
-        sink = guarded_region(instrs, live_out, fixed) if live_out is not None else None
+        sink = guarded_region(instrs, live_out, fixed, arms) if live_out is not None else None
         if sink:
             cond, inside = sink
             for p in todo:

@@ -1,0 +1,153 @@
+"""Blocks as the generator emits them, all its rules together: random blocks
+in which the arms of selects, work behind a condition and selections among
+constants meet, compiled for the CPU in the emitted order and in program
+order, leave the same live values (CPU)."""
+
+import ctypes
+import random
+import re
+import subprocess
+
+import numpy as np
+import pytest
+
+from loom_b200.codegen import emit_cuda as E
+from loom_b200.codegen import ir
+
+# registers 0-3: u64, 4-7: u32, 8-11: f32
+TYPES = ["u64"] * 4 + ["u32"] * 4 + ["f32"] * 4
+SIZE = {"u64": 8, "u32": 4, "f32": 4}
+HEAD = "loomir 1\nkernel t\nindex u32\nstraight 1\n" + "".join(f"reg {i} x{i} {SIZE[t]} {t}\n" for i, t in enumerate(TYPES))
+
+PRELUDE = r"""
+#include <cmath>
+#include <cstring>
+template <typename To, typename From> static To bitcast(From v) { static_assert(sizeof(To) == sizeof(From)); To r; memcpy(&r, &v, sizeof r); return r; }
+template <typename T> static T op_min(T a, T b) { return b < a ? b : a; }
+static float op_sqrt(float v) { return std::sqrt(v); }
+static bool op_differs(unsigned long long v, unsigned lit) { return v != lit; }
+#define __constant__ static const
+struct uint4 { unsigned x, y, z, w; };
+struct Regs { unsigned long long r0, r1, r2, r3; unsigned r4, r5, r6, r7; float r8, r9, r10, r11; };
+"""
+
+PTX = {"add.u64": "+", "sub.u64": "-", "mul.lo.u64": "*", "and.b64": "&", "or.b64": "|", "xor.b64": "^"}
+
+
+def _host(lines):
+    """The emitted lines with each inline-assembly statement as C++."""
+    out = []
+    it = iter(lines)
+    for ln in it:
+        if "asm(" not in ln:
+            out.append(ln)
+            continue
+        args = next(it)
+        sense, text = re.search(r"setp\.(eq|ne)\.u32 p, %1, 0; (.*)}\"", ln).groups()
+        cond = re.search(r'"r"\((.*?)\)(?:, "l"|\);)', args).group(1)
+        regs = re.findall(r'"l"\((R\.r\d+)\)', args)
+        at = {"%0": "v", **{f"%{2 + i}": f"a{i}" for i in range(len(regs))}}
+        out.append("{ " + " ".join(f"const unsigned long long a{i} = {r};" for i, r in enumerate(regs)))
+        out.append(f"if(({cond}) {'==' if sense == 'eq' else '!='} 0u) {{ unsigned long long t0, t1, t2, t3, t4; (void)t0; (void)t1; (void)t2; (void)t3; (void)t4;")
+        for op in re.findall(r"@p ([^;]*);", text):
+            name, rest = op.split(" ", 1)
+            d, *a = [at.get(x.strip(), x.strip() + ("ull" if x.strip().startswith("0x") else "")) for x in rest.split(",")]
+            out.append(f"{d} = {a[0]} * {a[1]} + {a[2]};" if name == "mad.lo.u64" else f"{d} = {a[0]} {PTX[name]} {a[1]};")
+        out.append("} }")
+    return out
+
+
+def _reg(rng, t):
+    lo = TYPES.index(t)
+    return f"r{rng.randrange(lo, lo + 4)}:{t}"
+
+
+def _operand(rng, t):
+    if t != "f32" and rng.random() < 0.15:
+        return f"k{t}:{rng.choice([0, 1, 2, 3]):#x}"
+    return _reg(rng, t)
+
+
+def _line(rng, constants):
+    u, f, w = (lambda t=t: _operand(rng, t) for t in ("u32", "f32", "u64"))
+    kind = rng.choice(["w", "w", "sel", "cmp", "cmp", "land", "f", "f", "root", "fsel", "fsel", "wsel"] + ["sct"] * (2 * constants))
+    if kind == "w":
+        return f"i {rng.choice(['mul', 'mul', 'add', 'sub', 'bxor'])} u64 {_reg(rng, 'u64')} {w()} {w()}"
+    if kind == "sel":
+        return f"i cmov - {_reg(rng, 'u64')} {u()} {w()} {w()}"
+    if kind == "cmp":
+        return f"i {rng.choice(['gt', 'lt'])} f32 {_reg(rng, 'u32')} {f()} {f()}"
+    if kind == "land":
+        d = _reg(rng, "u32")
+        return f"i pacc f32,u32,land,lt {d} {d} {f()} {f()}"
+    if kind == "f":
+        return f"i {rng.choice(['add', 'mul', 'div', 'div'])} f32 {_reg(rng, 'f32')} {f()} {f()}"
+    if kind == "root":
+        return f"i sqrt f32 {_reg(rng, 'f32')} {f()}"
+    if kind == "fsel":
+        d = _reg(rng, "f32")
+        return f"i cmov - {d} {u()} {f()} {d}"
+    if kind == "wsel":
+        d = _reg(rng, "u64")
+        return f"i cmov - {d} {u()} {w()} {d}"
+    t = rng.choice(["f32", "u32"])
+    return f"i sct {t},u32 {_reg(rng, t)} r4:u32 | " + " ".join(f"k{t}:{rng.choice([0, 1, 5, 0x3f800000, 0x40400000]):#x}" for _ in range(3))
+
+
+def _block(rng, constants):
+    """Lines of a block: random ones, and between some of them the form in
+    which the rules meet: an arm, a condition, the arm's select, then work
+    under the condition that may write what the arm reads."""
+    out = [_line(rng, constants) for _ in range(rng.randint(0, 6))]
+    if rng.random() < 0.8:
+        t, a, b, s = (_reg(rng, "u64") for _ in range(4))
+        h, g = _reg(rng, "u32"), _operand(rng, "u32")
+        x, y, z = (_reg(rng, "f32") for _ in range(3))
+        form = [f"i {rng.choice(['mul', 'add'])} u64 {t} {a} {b}", f"i lt f32 {h} {x} {y}",
+                f"i cmov - {s} {g} {t} {a}" if rng.random() < 0.5 else f"i cmov - {s} {g} {a} {t}",
+                f"i sqrt f32 {z} {x}", f"i div f32 {z} {z} {y}", f"i cmov - {y} {h} {z} {y}", f"i cmov - {b} {h} {a} {b}"]
+        for ln in form:
+            out.append(ln)
+            if rng.random() < 0.15:
+                out.append(_line(rng, constants))
+    return out + [_line(rng, constants) for _ in range(rng.randint(0, 4))]
+
+
+@pytest.mark.parametrize("constants", [False])
+def test_emitted_order_of_random_blocks(constants, tmp_path):
+    rng = random.Random(23 + constants)
+    src, lives, both = [PRELUDE], [], 0
+    for n in range(700):
+        lines = _block(rng, constants)
+        live = sorted(rng.sample(range(12), rng.randint(2, 5)))
+        k = ir.parse(HEAD + f"output {live[0]} {TYPES[live[0]]} o\nblock 0 START {len(lines)}\n" + "\n".join(lines) + "\nend\n")
+        L = E.Lowering(k, device=True)
+        ins = k.blocks[0].instrs
+        arms = E.select_arms(ins, set(live), dict(enumerate(TYPES)))
+        emitted = _host(L.body(ins, "", set(live), n))
+        both += bool(arms) and any(re.match(r"\s*if\(R\.", ln) for ln in emitted)
+        k.blocks[0].idx = n  # the constants' names
+        src += L.constant_tables(k.blocks[0])
+        src += [f'extern "C" void want{n}(Regs& R) {{', *(L.write(i.dst, L.expr(i)) for i in ins), "}"]
+        src += [f'extern "C" void got{n}(Regs& R) {{', *emitted, "}"]
+        lives.append((live, lines))
+    (tmp_path / "b.cpp").write_text("\n".join(src))
+    so = tmp_path / "b.so"
+    r = subprocess.run(["g++", "-std=c++17", "-O0", "-w", "-ffp-contract=off", "-shared", "-fPIC", "-o", so, tmp_path / "b.cpp"],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[:2000]
+    lib = ctypes.CDLL(str(so))
+    rng = np.random.default_rng(5)
+    fields = np.dtype([(f"r{i}", {"u64": "u8", "u32": "u4", "f32": "f4"}[t]) for i, t in enumerate(TYPES)], align=True)
+    for n, (live, lines) in enumerate(lives):
+        for _ in range(8):
+            v = np.zeros(1, fields)
+            for i, t in enumerate(TYPES):
+                v[f"r{i}"] = rng.choice([-1.0, 0.5, 2.0, 9.0]) if t == "f32" else rng.choice([0, 1, 2, 7]) if t == "u32" else rng.integers(0, 1 << 40)
+            want, got = v.copy(), v.copy()
+            getattr(lib, f"want{n}")(ctypes.c_void_p(want.ctypes.data))
+            getattr(lib, f"got{n}")(ctypes.c_void_p(got.ctypes.data))
+            for i in live:
+                a, b = want[f"r{i}"], got[f"r{i}"]
+                assert a.tobytes() == b.tobytes() or (a != a and b != b), (n, i, v, a, b, lines)
+    assert both > 60
