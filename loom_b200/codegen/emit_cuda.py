@@ -283,13 +283,14 @@ def predicated_ptx(arm):
     return " ".join(text), regs
 
 
-def select_arms(instrs, live_out, storage) -> Dict[int, tuple]:
+def select_arms(instrs, live_out, storage, barred=frozenset()) -> Dict[int, tuple]:
     """Selects of 64-bit integers whose operands are computed for them alone:
     {position of the cmov: (positions of the arm that runs in line, positions
     of the arm predicated over its result, whether that is the second
     value)}.  A 64-bit select costs two instructions on the ALU pipe, which
     bounds integer loops; with one arm predicated there is none (Collatz, a
-    warp's iteration with all lanes busy: 17.2 -> 13.2 cycles)."""
+    warp's iteration with all lanes busy: 17.2 -> 13.2 cycles).  Positions in
+    `barred` (members of constant rows, emitted as such) join no arm."""
     n = len(instrs)
     reach: Dict[int, int] = {}  # register -> position of its last definition
     uses: Dict[int, List[tuple]] = {}  # definition -> [(position, operand)]
@@ -316,7 +317,7 @@ def select_arms(instrs, live_out, storage) -> Dict[int, tuple]:
             while grown:
                 grown = False
                 for p in range(q):
-                    if p in arm or p in taken or p in kept or not isinstance(instrs[p], Compute):
+                    if p in arm or p in taken or p in kept or p in barred or not isinstance(instrs[p], Compute):
                         continue
                     if instrs[p].op in OP_COST or instrs[p].op in ("assert_fp", "tab", "cmov"):
                         continue
@@ -724,7 +725,8 @@ class Lowering:
             return out
 
         todo = [p for p, ins in enumerate(instrs) if isinstance(ins, Compute)]
-        arms = select_arms(instrs, live_out, {i: r.storage for i, r in self.regs.items()}) if live_out is not None else {}
+        storage = {i: r.storage for i, r in self.regs.items()}
+        arms = select_arms(instrs, live_out, storage, sct_of) if live_out is not None else {}
         in_arm = {p for a, b, _ in arms.values() for p in a + b}
         todo = [p for p in todo if p not in in_arm]
         out = []

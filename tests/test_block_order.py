@@ -110,10 +110,16 @@ def _block(rng, constants):
             out.append(ln)
             if rng.random() < 0.15:
                 out.append(_line(rng, constants))
+    if constants and rng.random() < 0.5:
+        # a row of three selections, one of which may feed one arm alone
+        sct = [f"i sct u32,u32 r{r}:u32 r4:u32 | ku32:0x1 ku32:{rng.randrange(9):#x} ku32:0x3" for r in (5, 6, 7)]
+        t, a, b, s = (_reg(rng, "u64") for _ in range(4))
+        rng.shuffle(sct)
+        out += sct + [f"i mov - {t} r{rng.choice([5, 6, 7])}:u32", f"i mul u64 {a} {a} {b}", f"i cmov - {s} r4:u32 {t} {a}"]
     return out + [_line(rng, constants) for _ in range(rng.randint(0, 4))]
 
 
-@pytest.mark.parametrize("constants", [False])
+@pytest.mark.parametrize("constants", [False, True])
 def test_emitted_order_of_random_blocks(constants, tmp_path):
     rng = random.Random(23 + constants)
     src, lives, both = [PRELUDE], [], 0
