@@ -680,7 +680,8 @@ class Lowering:
             if pos in sct:
                 idx, n, ps = sct[pos]
                 width = (len(ps) + 3) // 4
-                ct = CTYPE[idx.type]
+                # 8 and 16 bits need not hold the last entry's number
+                ct = CTYPE["u64" if idx.type == "u64" else "u32"]
                 out.append(indent + f"const uint4* sp{pos} = kSct{block}_{pos} + {width}u * static_cast<unsigned>(op_min<{ct}>({self.read(idx)}, {n - 1}));")
                 out.extend(indent + f"const uint4 sv{pos}_{j} = sp{pos}[{j}];" for j in range(width))
             if pos in sct_of:

@@ -157,3 +157,31 @@ def test_emitted_order_of_random_blocks(constants, tmp_path):
                 a, b = want[f"r{i}"], got[f"r{i}"]
                 assert a.tobytes() == b.tobytes() or (a != a and b != b), (n, i, v, a, b, lines)
     assert both > 60
+
+
+@pytest.mark.parametrize("t", ["u8", "u16", "u32", "u64"])
+@pytest.mark.parametrize("entries", [3, 256, 257, 300])
+def test_index_types_of_constant_rows(t, entries, tmp_path):
+    """Every index value takes its own entry, those from the last on the last,
+    also where the index's type does not hold the number of entries."""
+    n = ir.TYPE_BYTES[t]
+    head = f"loomir 1\nkernel t\nindex u32\nstraight 1\nreg 0 i {n} {t}\n" + "".join(f"reg {r} x{r} 4 u32\n" for r in (1, 2, 3))
+    lines = [f"i sct u32,{t} r{r}:u32 r0:{t} | " + " ".join(f"ku32:{e * 4 + r:#x}" for e in range(entries)) for r in (1, 2, 3)]
+    k = ir.parse(head + f"input 0 {t} i\noutput 1 u32 x1\nblock 0 START 3\n" + "\n".join(lines) + "\nend\n")
+    L = E.Lowering(k, device=True)
+    b = k.blocks[0]
+    assert len(L.constant_rows(b.instrs)) == 1
+    ct = {1: "unsigned char", 2: "unsigned short", 4: "unsigned", 8: "unsigned long long"}[n]
+    code = PRELUDE.replace("struct Regs", "struct Unused") + "\n".join(L.constant_tables(b)) + f"\nstruct Regs {{ {ct} r0; unsigned r1, r2, r3; }};\n"
+    code += f'extern "C" void run({ct} i, unsigned* o) {{ Regs R{{i, 0, 0, 0}};\n' + "\n".join(L.body(b.instrs, "", {1, 2, 3}, 0)) + "\no[0] = R.r1; o[1] = R.r2; o[2] = R.r3; }"
+    (tmp_path / "c.cpp").write_text(code)
+    r = subprocess.run(["g++", "-std=c++17", "-O0", "-w", "-shared", "-fPIC", "-o", tmp_path / "c.so", tmp_path / "c.cpp"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[:2000]
+    lib = ctypes.CDLL(str(tmp_path / "c.so"))
+    arg = {1: ctypes.c_uint8, 2: ctypes.c_uint16, 4: ctypes.c_uint32, 8: ctypes.c_uint64}[n]
+    out = (ctypes.c_uint32 * 3)()
+    for i in sorted({0, 1, 2, 43, 44, 45, 127, 254, 255, 256, 257, 299, 300, 65535, 1 << 31, (1 << 32) + 1, (1 << 64) - 1}):
+        if i >> (8 * n):
+            continue
+        lib.run(arg(i), out)
+        assert list(out) == [min(i, entries - 1) * 4 + r for r in (1, 2, 3)], i
