@@ -470,6 +470,12 @@ def guarded_region(instrs, live_out, fixed, arms=None):
 # 51.4 ms.
 SCT_MIN = 3
 
+# Bytes of a kernel's constant rows, at most: constant memory holds 65536, of
+# which the engine's own tables take 8 a block.  The largest selections of
+# Loom's path tracers take 560 bytes a kernel.  What does not fit stays a
+# chain of selects.
+SCT_BYTES = 48 << 10
+
 
 class Lowering:
     def __init__(self, k: Kernel, device: bool = False):
@@ -480,6 +486,15 @@ class Lowering:
         # lowers with this class too, without the device's helpers)
         self.device = device
         self.mad_adds = False
+        # (block, first position) of the constant rows that fit
+        self.rows_kept = set()
+        left = SCT_BYTES
+        for b in k.blocks:
+            for first, (_, n, ps) in self.constant_rows(b.instrs).items():
+                size = n * ((len(ps) + 3) // 4) * 16
+                if size <= left:
+                    left -= size
+                    self.rows_kept.add((b.idx, first))
 
     # ------------------------------------------------------------ views
     def rname(self, idx: int) -> str:
@@ -633,11 +648,12 @@ class Lowering:
                 member[p] = (first, d)
         return rows, member
 
-    def constant_rows(self, instrs):
+    def constant_rows(self, instrs, block=None):
         """Selections among constants (`sct`) by one index: {position of the
         first: (index operand, entries, positions)} of every SCT_MIN or more
         of them on an index that does not change in between, with the same
-        number of 4-byte entries."""
+        number of 4-byte entries.  With the number of the block: those of
+        them that constant memory has room for."""
         groups: Dict[tuple, List[int]] = {}
         version: Dict[int, int] = {}
         for p, ins in enumerate(instrs):
@@ -650,13 +666,14 @@ class Lowering:
             ):
                 groups.setdefault((a.reg, version.get(a.reg, 0), len(ins.consts)), []).append(p)
             version[ins.dst.reg] = version.get(ins.dst.reg, 0) + 1
-        return {ps[0]: (instrs[ps[0]].args[0], n, ps) for (_, _, n), ps in groups.items() if len(ps) >= SCT_MIN}
+        rows = {ps[0]: (instrs[ps[0]].args[0], n, ps) for (_, _, n), ps in groups.items() if len(ps) >= SCT_MIN}
+        return {p: r for p, r in rows.items() if block is None or (block, p) in self.rows_kept}
 
     def constant_tables(self, blk) -> List[str]:
         """Definitions of a block's constant rows: an entry's values side by
         side, padded to whole 16-byte words."""
         out = []
-        for first, (_, n, ps) in self.constant_rows(blk.instrs).items():
+        for first, (_, n, ps) in self.constant_rows(blk.instrs, blk.idx).items():
             rows = []
             for i in range(n):
                 words = [f"{blk.instrs[p].consts[i].bits & 0xFFFFFFFF:#x}u" for p in ps]
@@ -671,7 +688,7 @@ class Lowering:
         needs to move behind it."""
         rows, member = self.table_rows(instrs)
 
-        sct = self.constant_rows(instrs)
+        sct = self.constant_rows(instrs, block)
         sct_of = {p: (first, j) for first, (_, _, ps) in sct.items() for j, p in enumerate(ps)}
 
         def emit(pos: int, indent: str) -> List[str]:

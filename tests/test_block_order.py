@@ -127,12 +127,12 @@ def test_emitted_order_of_random_blocks(constants, tmp_path):
         lines = _block(rng, constants)
         live = sorted(rng.sample(range(12), rng.randint(2, 5)))
         k = ir.parse(HEAD + f"output {live[0]} {TYPES[live[0]]} o\nblock 0 START {len(lines)}\n" + "\n".join(lines) + "\nend\n")
+        k.blocks[0].idx = n  # the constants' names
         L = E.Lowering(k, device=True)
         ins = k.blocks[0].instrs
         arms = E.select_arms(ins, set(live), dict(enumerate(TYPES)))
         emitted = _host(L.body(ins, "", set(live), n))
         both += bool(arms) and any(re.match(r"\s*if\(R\.", ln) for ln in emitted)
-        k.blocks[0].idx = n  # the constants' names
         src += L.constant_tables(k.blocks[0])
         src += [f'extern "C" void want{n}(Regs& R) {{', *(L.write(i.dst, L.expr(i)) for i in ins), "}"]
         src += [f'extern "C" void got{n}(Regs& R) {{', *emitted, "}"]
@@ -185,3 +185,24 @@ def test_index_types_of_constant_rows(t, entries, tmp_path):
             continue
         lib.run(arg(i), out)
         assert list(out) == [min(i, entries - 1) * 4 + r for r in (1, 2, 3)], i
+
+
+def _wide(entries, groups):
+    """A kernel of `groups` blocks of four selections of `entries` each."""
+    blocks = [f"block {b} b{b} 5\n" + "".join(f"i sct u32,u32 r{r}:u32 r0:u32 | " + " ".join(f"ku32:{e * b + r:#x}" for e in range(entries)) + "\n"
+              for r in (1, 2, 3, 4)) + f"j {b + 1 if b + 1 < groups else -1}\n" for b in range(groups)]
+    head = "loomir 1\nkernel t\nindex u32\nstraight 0\n" + "".join(f"reg {r} x{r} 4 u32\n" for r in range(5))
+    return ir.parse(head + "input 0 u32 x0\noutput 1 u32 x1\n" + "".join(blocks) + "end\n")
+
+
+@pytest.mark.parametrize("entries,groups,kept", [(3, 2, [0, 1]), (3072, 1, [0]), (3073, 1, []), (1024, 4, [0, 1, 2]), (2000, 2, [0]), (12000, 2, [])])
+def test_constant_rows_that_fit_constant_memory(entries, groups, kept):
+    """Rows beyond the kernel's share of constant memory stay selects."""
+    k = _wide(entries, groups)
+    L = E.Lowering(k, device=True)
+    tables = [t for b in k.blocks for t in L.constant_tables(b)]
+    assert [int(re.search(r"kSct(\d+)_0\[", t).group(1)) for t in tables] == kept
+    assert sum(16 * int(re.search(r"\[(\d+)\]", t).group(1)) for t in tables) <= 49152
+    for b in k.blocks:
+        body = "\n".join(L.body(b.instrs, "", {1, 2, 3, 4}, b.idx))
+        assert ("kSct" in body) == (b.idx in kept) and (" ? " in body) == (b.idx not in kept)
