@@ -570,8 +570,9 @@ class Lowering:
             # on the halves that sets the predicate, instead of a compare of
             # each half (the ALU pipe takes two cycles for either)
             for i, lit in ((0, ins.args[1]), (1, ins.args[0])):
-                if lit.is_literal and not ins.args[i].is_literal and lit.value() in range(1 << 32):
-                    return f"{'' if op == 'ne' else '!'}op_differs({cv(i, 'u64')}, {lit.value():#x}u)"
+                if lit.is_literal and lit.type in INT_TYPES and not ins.args[i].is_literal and lit.value() in range(1 << 32):
+                    v = f"static_cast<{CTYPE['u64']}>({cv(i, t)})"
+                    return f"{'' if op == 'ne' else '!'}op_differs({v}, {lit.value():#x}u)"
         if op in CMP:
             return f"static_cast<bool>({cv(0, t)} {CMP[op]} {cv(1, t)})"
         if op in LOGIC:

@@ -153,7 +153,7 @@ struct K
                 R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
             }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1)), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
@@ -166,7 +166,7 @@ struct K
                 R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
             }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1)), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
@@ -179,7 +179,7 @@ struct K
                 R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
             }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1)), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
@@ -192,7 +192,7 @@ struct K
                 R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
             }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1)), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
@@ -205,7 +205,7 @@ struct K
                 R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
             }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1)), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
@@ -218,7 +218,7 @@ struct K
                 R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
             }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1)), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
@@ -231,7 +231,7 @@ struct K
                 R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
             }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1)), 0x1u));
             if(!(R.r3)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 1, 8u);
@@ -244,7 +244,7 @@ struct K
                 R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
             }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1)), 0x1u));
             if(!(R.r3)) goto L_HALT;
             left -= 8u;
         }
@@ -261,7 +261,7 @@ struct K
                 R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(v));
             }
             R.r2 = static_cast<unsigned int>(static_cast<unsigned int>(static_cast<unsigned int>(R.r2) + static_cast<unsigned int>(((unsigned int)0x1ull))));
-            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(R.r1), 0x1u));
+            R.r3 = static_cast<unsigned long long>(op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1)), 0x1u));
             --left;
             if(!(R.r3)) goto L_HALT;
         }

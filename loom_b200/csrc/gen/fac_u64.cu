@@ -149,49 +149,49 @@ struct K
             if constexpr(kProf) count_block(ctx, 2, 4u);
             R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
             R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(R.r3), 0x0u));
+            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3)), 0x0u));
             if(!!(R.r2)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 2, 4u);
             R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
             R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(R.r3), 0x0u));
+            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3)), 0x0u));
             if(!!(R.r2)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 2, 4u);
             R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
             R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(R.r3), 0x0u));
+            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3)), 0x0u));
             if(!!(R.r2)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 2, 4u);
             R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
             R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(R.r3), 0x0u));
+            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3)), 0x0u));
             if(!!(R.r2)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 2, 4u);
             R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
             R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(R.r3), 0x0u));
+            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3)), 0x0u));
             if(!!(R.r2)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 2, 4u);
             R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
             R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(R.r3), 0x0u));
+            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3)), 0x0u));
             if(!!(R.r2)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 2, 4u);
             R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
             R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(R.r3), 0x0u));
+            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3)), 0x0u));
             if(!!(R.r2)) goto L_HALT;
             fresh = false;
             if constexpr(kProf) count_block(ctx, 2, 4u);
             R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
             R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(R.r3), 0x0u));
+            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3)), 0x0u));
             if(!!(R.r2)) goto L_HALT;
             left -= 8u;
         }
@@ -201,7 +201,7 @@ struct K
             if constexpr(kProf) count_block(ctx, 2, 4u);
             R.r1 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r1) * static_cast<unsigned long long>(R.r3)));
             R.r3 = static_cast<unsigned long long>(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3) - static_cast<unsigned long long>(((unsigned long long)0x1ull))));
-            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(R.r3), 0x0u));
+            R.r2 = static_cast<unsigned long long>(!op_differs(static_cast<unsigned long long>(static_cast<unsigned long long>(R.r3)), 0x0u));
             --left;
             if(!!(R.r2)) goto L_HALT;
         }
