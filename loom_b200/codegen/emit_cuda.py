@@ -87,6 +87,15 @@ def long_blocks(k: Kernel) -> List[int]:
     return sorted((b for b in range(k.num_blocks) if counts[b] >= LONG_BLOCK_INSTR), key=lambda b: -counts[b])[:4]
 
 
+def any_order(k: Kernel) -> bool:
+    """Whether schedule 2 needs no order among the blocks where lanes can
+    stand (block 0 and those where a step may end): one loop at most, and no
+    long block among several, for which lanes may have to wait."""
+    steps = k.step_headers(set(long_blocks(k)))
+    stands = steps | {0}
+    return len(steps) <= 1 and (len(stands) == 1 or not stands & set(long_blocks(k)))
+
+
 # Copies of a block that loops on itself: (most instructions, copies with an
 # exit each, copies of a counted loop without).  A look at the iterations left, the loop's condition and its counter cost as
 # much as a short body.  Copies with one look per group: 2^20 Fibonacci
@@ -924,7 +933,7 @@ def generate(k: Kernel) -> str:
     w(f"    static constexpr int kRegroupMaxRegs = {REGROUP_MAX_REGS};")
     # small kernels: two inlined copies of their code in the megakernel
     w(f"    static constexpr bool kSplitCallSites = {'true' if sum(counts) <= REG_VARIANT_MIN_INSTR else 'false'};")
-    w(f"    static constexpr int kStepHeaders = {len(k.step_headers(set(long_blocks(k))))}; // blocks where a step may end")
+    w(f"    static constexpr bool kAnyOrder = {str(any_order(k)).lower()}; // schedule 2: lanes need no order")
     spread = bool(k.loop_headers()) and sum(counts) > REG_VARIANT_MIN_INSTR
     w(f"    static constexpr bool kSpread = {str(spread).lower()}; // a large program with loops")
     # kernels that read records of the table: their launches on flat tables

@@ -469,10 +469,11 @@ regroup_kernel(const RegroupParams p)
                         run = rk == lo;
                         if(run) --visits;
                     }
-                    else if(minpc && K::kStepHeaders <= 1)
+                    else if(minpc && K::kAnyOrder)
                     {
-                        // one loop: no order to keep, so no ranks to read
-                        // and no minimum to vote (Collatz, 2^24 threads 2.29
+                        // one loop, no long block to wait for: no order to
+                        // keep, so no ranks to read and no minimum to vote
+                        // (Collatz, 2^24 threads 2.29
                         // -> 2.03 ms; with two loops a ballot per block where
                         // lanes can stand was slower than the vote, 22.8 ->
                         // 23.2 ms on the 1024x768x64 render)

@@ -18,7 +18,7 @@ struct K
     static constexpr int kNumQueues = 3;
     static constexpr int kRegroupMaxRegs = 64;
     static constexpr bool kSplitCallSites = true;
-    static constexpr int kStepHeaders = 1; // blocks where a step may end
+    static constexpr bool kAnyOrder = true; // schedule 2: lanes need no order
     static constexpr bool kSpread = false; // a large program with loops
     static constexpr bool kTableRows = false;
     struct Regs

@@ -22,7 +22,7 @@ struct K
     static constexpr int kNumQueues = 55;
     static constexpr int kRegroupMaxRegs = 64;
     static constexpr bool kSplitCallSites = false;
-    static constexpr int kStepHeaders = 5; // blocks where a step may end
+    static constexpr bool kAnyOrder = false; // schedule 2: lanes need no order
     static constexpr bool kSpread = true; // a large program with loops
     static constexpr bool kTableRows = false;
     struct Regs

@@ -18,7 +18,7 @@ struct K
     static constexpr int kNumQueues = 28;
     static constexpr int kRegroupMaxRegs = 64;
     static constexpr bool kSplitCallSites = false;
-    static constexpr int kStepHeaders = 2; // blocks where a step may end
+    static constexpr bool kAnyOrder = false; // schedule 2: lanes need no order
     static constexpr bool kSpread = true; // a large program with loops
     static constexpr bool kTableRows = true;
     struct Regs
