@@ -1078,15 +1078,23 @@ def generate(k: Kernel) -> str:
     w("    // stopped at, or kHalt.  With `stop_heavy`, a block whose quorum is")
     w("    // above zero is entered only as the first block of the burst, when")
     w("    // the warp's vote chose it.  A block that loops on itself takes up")
-    w("    // to `spin` further iterations without spending budget (a loop the")
+    w("    // to `spin` iterations (not 0) for one of the budget (a loop the")
     w("    // warp's lanes run together needs no step of its own per iteration).")
     w("    // kFlat: the launch's table is flat (Columns::table_flat).  kAllHeaders:")
     w("    // every loop header spends budget (the plain engine's step guard);")
     w("    // otherwise a minimal set of them that every cycle passes.")
     w("    template <bool kProf, bool kFlat, bool kAllHeaders>")
     w("    __device__ __forceinline__ static int")
-    w("    run_burst(const int entry, Regs& R, Ctx& ctx, unsigned budget, const bool stop_heavy = false,")
+    w("    run_burst(const int entry, Regs& R, Ctx& ctx, const unsigned budget, const bool stop_heavy = false,")
     w("              unsigned spin = 0u)")
+    w("    {")
+    w("        return run_steps<kProf, kFlat, kAllHeaders>(entry, R, ctx, budget, stop_heavy, spin);")
+    w("    }")
+    w("    // ... which takes the iterations it ran off `spin` (programs of several")
+    w("    // loops; one loop's last iterations stay uncounted, as only HALT follows).")
+    w("    template <bool kProf, bool kFlat, bool kAllHeaders>")
+    w("    __device__ __forceinline__ static int")
+    w("    run_steps(const int entry, Regs& R, Ctx& ctx, unsigned budget, const bool stop_heavy, unsigned& spin)")
     w("    {")
     w("        (void)ctx;")
     w("        (void)stop_heavy;")
@@ -1129,8 +1137,9 @@ def generate(k: Kernel) -> str:
             if blk.terminator.targets[0] == b:
                 stay = f"!{stay}"
             other = next(t for t in blk.terminator.targets if t != b)
-            # a loop that only HALT can follow leaves the counters alone
-            ends = not (k.reachable(other) & headers)
+            # a loop that only HALT can follow leaves the counters alone (the
+            # ordered form of programs of several loops reads them)
+            ends = not (k.reachable(other) & headers) and len(steps) <= 1
             counted = counted_loop(blk)
             w(f"        if(budget == 0u) return {b};")
             w("        left = spin ? spin : budget;")
@@ -1182,6 +1191,8 @@ def generate(k: Kernel) -> str:
         if b in steps:
             w(f"        if(budget == 0u) return {b};")
             w("        --budget;")
+            if self_loop:
+                w("        if(spin) --spin;")
         elif b in headers:
             w(f"        if(kAllHeaders && budget == 0u) return {b};")
             w("        if(kAllHeaders) --budget;")

@@ -455,9 +455,10 @@ regroup_kernel(const RegroupParams p)
                 // of the chosen group `burst` visits; in programs of several
                 // loops the lanes take them in that same order (kOrdered)
                 // instead of each along its own path: a 320x240x16 render
-                // with default options 2.25 -> 1.04 ms.
-                const bool stepped = kOrdered || minpc;
-                unsigned   visits  = kOrdered && pc >= 0 && (mc >= p.spread || pc == m) ? p.burst : 0u;
+                // with default options 2.25 -> 1.10 ms (0.99 ms with loops
+                // run to their end within one visit, but then neither burst
+                // nor period bounds what a tile runs in a round).
+                unsigned visits = kOrdered && pc >= 0 && (mc >= p.spread || pc == m) ? p.burst : 0u;
                 for(unsigned i = 0; kOrdered || i < (minpc ? p.burst : 1u); ++i)
                 {
                     bool run;
@@ -467,16 +468,15 @@ regroup_kernel(const RegroupParams p)
                         const unsigned lo = __reduce_min_sync(FULL, rk);
                         if(lo == 0xffffffffu) break;
                         run = rk == lo;
-                        if(run) --visits;
                     }
                     else if(minpc && K::kAnyOrder)
                     {
                         // one loop, no long block to wait for: no order to
                         // keep, so no ranks to read and no minimum to vote
-                        // (Collatz, 2^24 threads 2.29
-                        // -> 2.03 ms; with two loops a ballot per block where
-                        // lanes can stand was slower than the vote, 22.8 ->
-                        // 23.2 ms on the 1024x768x64 render)
+                        // (Collatz, 2^24 threads 2.29 -> 2.03 ms; with two
+                        // loops a ballot per block where lanes can stand was
+                        // slower than the vote, 22.8 -> 23.2 ms on the
+                        // 1024x768x64 render)
                         run = pc >= 0;
                         if(__ballot_sync(FULL, run) == 0u) break;
                     }
@@ -496,7 +496,15 @@ regroup_kernel(const RegroupParams p)
                     }
                     else
                         run = pc >= 0 && (p.schedule == 3u || mc >= p.spread || pc == m);
-                    if(run)
+                    if constexpr(kOrdered)
+                    {
+                        // a lane may spend what it has left of the burst on
+                        // one loop; iterations count as visits do
+                        unsigned spin = visits;
+                        if(run) pc = K::template run_steps<kProf, kFlat, false>(pc, R, ctx, 1u, false, spin);
+                        if(run) visits = spin < visits ? spin : visits - 1u;
+                    }
+                    else if(run)
                     {
                         if constexpr(K::kSplitCallSites)
                         {
@@ -504,19 +512,19 @@ regroup_kernel(const RegroupParams p)
                             // call site: spin_iters picks 16, 64 or the
                             // default (a few iterations let halted lanes take
                             // new threads while the others keep looping)
-                            if(stepped && p.spin_iters && p.spin_iters <= 16u)
+                            if(minpc && p.spin_iters && p.spin_iters <= 16u)
                                 pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, 1u, false, 16u);
-                            else if(stepped && p.spin_iters && p.spin_iters <= 64u)
+                            else if(minpc && p.spin_iters && p.spin_iters <= 64u)
                                 pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, 1u, false, 64u);
-                            else if(stepped)
+                            else if(minpc)
                                 pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, 1u, false, kSelfLoopSpin);
                             else
                                 pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, p.burst, kPark && cost_on && p.schedule < 2u);
                         }
                         else
-                            pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, stepped ? 1u : p.burst,
+                            pc = K::template run_burst<kProf, kFlat, false>(pc, R, ctx, minpc ? 1u : p.burst,
                                                               kPark && cost_on && p.schedule < 2u,
-                                                              stepped ? (p.spin_iters ? p.spin_iters : kSelfLoopSpin) : 0u);
+                                                              minpc ? (p.spin_iters ? p.spin_iters : kSelfLoopSpin) : 0u);
                     }
                     // a burst also ends once a quarter of the lanes have
                     // halted, while there are inputs to replace them (1.05 ->

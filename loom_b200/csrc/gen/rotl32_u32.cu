@@ -104,15 +104,23 @@ struct K
     // stopped at, or kHalt.  With `stop_heavy`, a block whose quorum is
     // above zero is entered only as the first block of the burst, when
     // the warp's vote chose it.  A block that loops on itself takes up
-    // to `spin` further iterations without spending budget (a loop the
+    // to `spin` iterations (not 0) for one of the budget (a loop the
     // warp's lanes run together needs no step of its own per iteration).
     // kFlat: the launch's table is flat (Columns::table_flat).  kAllHeaders:
     // every loop header spends budget (the plain engine's step guard);
     // otherwise a minimal set of them that every cycle passes.
     template <bool kProf, bool kFlat, bool kAllHeaders>
     __device__ __forceinline__ static int
-    run_burst(const int entry, Regs& R, Ctx& ctx, unsigned budget, const bool stop_heavy = false,
+    run_burst(const int entry, Regs& R, Ctx& ctx, const unsigned budget, const bool stop_heavy = false,
               unsigned spin = 0u)
+    {
+        return run_steps<kProf, kFlat, kAllHeaders>(entry, R, ctx, budget, stop_heavy, spin);
+    }
+    // ... which takes the iterations it ran off `spin` (programs of several
+    // loops; one loop's last iterations stay uncounted, as only HALT follows).
+    template <bool kProf, bool kFlat, bool kAllHeaders>
+    __device__ __forceinline__ static int
+    run_steps(const int entry, Regs& R, Ctx& ctx, unsigned budget, const bool stop_heavy, unsigned& spin)
     {
         (void)ctx;
         (void)stop_heavy;
