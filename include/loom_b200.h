@@ -91,7 +91,9 @@ typedef struct loom_b200_opts
     uint32_t mode;        /* LOOM_B200_PLAIN or LOOM_B200_REGROUP */
     uint32_t block_size;  /* CUDA threads per CTA (multiple of 32; 0: 256, and
                              for plain launches the engine's own choice, one
-                             warp for kernels of many registers) */
+                             warp for kernels of many registers); a size that
+                             the kernel's registers do not allow runs as the
+                             largest smaller one that fits */
     uint32_t utr_lanes;   /* regroup: keep running in registers while the
                              largest same-PC group has >= utr_lanes lanes
                              (the GPU form of Loom's UTR, simd.hpp:3273-3292) */

@@ -1434,12 +1434,13 @@ def generate(k: Kernel) -> str:
     w("    return cudaLaunchKernel(fn, dim3(static_cast<unsigned>(grid)), dim3(a.block), args, 0, a.stream);")
     w("}")
     w("")
-    w("// registers of a thread of the plain kernel")
-    w("cudaError_t plain_regs(bool profile, bool flat, int* regs)")
+    w("// registers of a thread of the plain kernel, and the threads a CTA of it can have")
+    w("cudaError_t plain_attrs(bool profile, bool flat, unsigned per, int* regs, int* max_threads)")
     w("{")
     w("    cudaFuncAttributes  at{};")
-    w("    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat, 1u));")
-    w("    *regs = at.numRegs;")
+    w("    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat, per));")
+    w("    *regs        = at.numRegs;")
+    w("    *max_threads = at.maxThreadsPerBlock;")
     w("    return e;")
     w("}")
     w("")
@@ -1516,7 +1517,7 @@ def generate(k: Kernel) -> str:
     w(f"    &loom_b200::k_{name}::kInfo, loom_b200::k_{name}::K::kRowBytes, {nq},")
     w(f"    &loom_b200::k_{name}::launch_plain, &loom_b200::k_{name}::launch_regroup,")
     w(f"    &loom_b200::k_{name}::regroup_occupancy,")
-    w(f"    &loom_b200::k_{name}::plain_regs,")
+    w(f"    &loom_b200::k_{name}::plain_attrs,")
     w(f"    loom_b200::k_{name}::kQueues, loom_b200::k_{name}::kSegments,")
     w(f"    loom_b200::k_{name}::kRegCaps, {len(caps)}u, loom_b200::k_{name}::K::kMaxStageRow, loom_b200::k_{name}::K::kSpread, {"loom_b200::kStraightPer" if several else "1u"}}};")
     return "\n".join(o) + "\n"

@@ -5958,12 +5958,13 @@ cudaError_t launch_plain(const PlainLaunch& a)
     return cudaLaunchKernel(fn, dim3(static_cast<unsigned>(grid)), dim3(a.block), args, 0, a.stream);
 }
 
-// registers of a thread of the plain kernel
-cudaError_t plain_regs(bool profile, bool flat, int* regs)
+// registers of a thread of the plain kernel, and the threads a CTA of it can have
+cudaError_t plain_attrs(bool profile, bool flat, unsigned per, int* regs, int* max_threads)
 {
     cudaFuncAttributes  at{};
-    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat, 1u));
-    *regs = at.numRegs;
+    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat, per));
+    *regs        = at.numRegs;
+    *max_threads = at.maxThreadsPerBlock;
     return e;
 }
 
@@ -6049,6 +6050,6 @@ const loom_b200::KernelEntry loom_b200_entry_primary_const_b20_256 = {
     &loom_b200::k_primary_const_b20_256::kInfo, loom_b200::k_primary_const_b20_256::K::kRowBytes, 33,
     &loom_b200::k_primary_const_b20_256::launch_plain, &loom_b200::k_primary_const_b20_256::launch_regroup,
     &loom_b200::k_primary_const_b20_256::regroup_occupancy,
-    &loom_b200::k_primary_const_b20_256::plain_regs,
+    &loom_b200::k_primary_const_b20_256::plain_attrs,
     loom_b200::k_primary_const_b20_256::kQueues, loom_b200::k_primary_const_b20_256::kSegments,
     loom_b200::k_primary_const_b20_256::kRegCaps, 8u, loom_b200::k_primary_const_b20_256::K::kMaxStageRow, loom_b200::k_primary_const_b20_256::K::kSpread, 1u};

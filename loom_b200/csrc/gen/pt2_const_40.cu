@@ -15194,12 +15194,13 @@ cudaError_t launch_plain(const PlainLaunch& a)
     return cudaLaunchKernel(fn, dim3(static_cast<unsigned>(grid)), dim3(a.block), args, 0, a.stream);
 }
 
-// registers of a thread of the plain kernel
-cudaError_t plain_regs(bool profile, bool flat, int* regs)
+// registers of a thread of the plain kernel, and the threads a CTA of it can have
+cudaError_t plain_attrs(bool profile, bool flat, unsigned per, int* regs, int* max_threads)
 {
     cudaFuncAttributes  at{};
-    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat, 1u));
-    *regs = at.numRegs;
+    const cudaError_t e = cudaFuncGetAttributes(&at, plain_fn(profile, flat, per));
+    *regs        = at.numRegs;
+    *max_threads = at.maxThreadsPerBlock;
     return e;
 }
 
@@ -15285,6 +15286,6 @@ const loom_b200::KernelEntry loom_b200_entry_pt2_const_40 = {
     &loom_b200::k_pt2_const_40::kInfo, loom_b200::k_pt2_const_40::K::kRowBytes, 55,
     &loom_b200::k_pt2_const_40::launch_plain, &loom_b200::k_pt2_const_40::launch_regroup,
     &loom_b200::k_pt2_const_40::regroup_occupancy,
-    &loom_b200::k_pt2_const_40::plain_regs,
+    &loom_b200::k_pt2_const_40::plain_attrs,
     loom_b200::k_pt2_const_40::kQueues, loom_b200::k_pt2_const_40::kSegments,
     loom_b200::k_pt2_const_40::kRegCaps, 8u, loom_b200::k_pt2_const_40::K::kMaxStageRow, loom_b200::k_pt2_const_40::K::kSpread, 1u};

@@ -305,6 +305,9 @@ struct loom_b200_handle
 
     bool     own_block    = true; // the plain engine picks its CTA size
     unsigned plain_blk[2] = {0, 0}; // its choice, by whether the table is flat (0: not made yet)
+    // threads a CTA of the plain kernel can have: [profiled][flat][several
+    // Loom threads per CUDA thread] (0: not asked yet)
+    unsigned plain_max[2][2][2] = {};
 
     loom_b200_stats stats{};
     unsigned        last_grid     = 0;
@@ -502,7 +505,8 @@ plain_block(loom_b200_handle* h, PlainLaunch& L)
     if(blk == 0)
     {
         int regs = 0;
-        LB_CUDA(h->e->plain_regs(false, flat, &regs));
+        int max  = 0;
+        LB_CUDA(h->e->plain_attrs(false, flat, 1u, &regs, &max));
         blk = regs >= kOneWarpRegs ? 32u : kDefaultPlainBlock;
     }
     L.block = blk;
@@ -511,6 +515,35 @@ plain_block(loom_b200_handle* h, PlainLaunch& L)
         const unsigned long long warps = static_cast<unsigned long long>(h->sms) * kSpreadWarps;
         while(L.lanes > 1u && L.n <= L.lanes / 2u * warps) L.lanes /= 2u;
     }
+    return LOOM_B200_OK;
+}
+
+/// The largest CTA size up to the named one that the kernel's registers allow
+/// (up to the default size they always do).
+int
+plain_fit(loom_b200_handle* h, PlainLaunch& L)
+{
+    auto most = [&](const unsigned per, unsigned& threads) -> cudaError_t
+    {
+        unsigned& m = h->plain_max[L.profile][L.cols.table_flat != 0u][per > 1u];
+        if(m == 0)
+        {
+            int               regs = 0, max = 0;
+            const cudaError_t rc   = h->e->plain_attrs(L.profile, L.cols.table_flat != 0u, per, &regs, &max);
+            if(rc != cudaSuccess) return rc;
+            m = static_cast<unsigned>(max);
+        }
+        threads = m;
+        return cudaSuccess;
+    };
+    if(L.block <= kDefaultPlainBlock) return LOOM_B200_OK;
+    unsigned threads = 0;
+    LB_CUDA(most(L.per, threads));
+    if(L.block <= threads) return LOOM_B200_OK;
+    // one Loom thread per CUDA thread takes fewer registers
+    L.per = 1u;
+    LB_CUDA(most(1u, threads));
+    L.block = std::min(L.block, threads / 32u * 32u);
     return LOOM_B200_OK;
 }
 
@@ -677,6 +710,8 @@ launch(loom_b200_handle* h, const loom_b200_launch& L, cudaStream_t stream, uint
             const int rc = plain_block(h, L);
             if(rc) return rc;
         }
+        const int rc = plain_fit(h, L);
+        if(rc) return rc;
         LB_CUDA(e.plain(L));
         const uint64_t cta = L.lanes < 32u ? L.lanes : static_cast<uint64_t>(L.block) * L.per;
         h->last_grid       = static_cast<unsigned>((n + cta - 1) / cta);

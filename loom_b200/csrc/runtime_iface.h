@@ -95,7 +95,8 @@ struct KernelEntry
     cudaError_t (*regroup)(const RegroupLaunch&);
     cudaError_t (*regroup_occupancy)(int block, bool profile, unsigned regs, unsigned dyn_smem, RegroupForm form,
                                      bool flat, int* ctas_per_sm);
-    cudaError_t (*plain_regs)(bool profile, bool flat, int* regs); // registers per thread of the plain kernel
+    // registers per thread of the plain kernel, and the threads a CTA of it can have
+    cudaError_t (*plain_attrs)(bool profile, bool flat, unsigned per, int* regs, int* max_threads);
     const loom_b200_queue_layout* queues;   // num_queues entries
     const QueueSegment*           segments; // num_queues entries
     const unsigned*               reg_caps; // compiled register caps, default first
