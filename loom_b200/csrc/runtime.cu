@@ -495,13 +495,15 @@ launch_graph(loom_b200_handle* h, const RegroupLaunch& L, uint64_t admit, cudaSt
 /// kernels (path tracers) differ by large factors: 512x512 pixels of Loom's
 /// pt_const 70.0 -> 61.9 ms with CTAs of one warp, a 320x240x16 sphere render
 /// 3.08 -> 2.81 ms; kernels of few registers lose (2^20 Fibonacci threads 24
-/// -> 32 us) as half their warps do not fit.
+/// -> 32 us) as half their warps do not fit.  Profiled launches take the size
+/// of the launch they describe (by the unprofiled kernel's registers); of the
+/// several Loom threads per CUDA thread of loop-free programs they run one,
+/// which puts the same threads together in a warp.
 int
 plain_block(loom_b200_handle* h, PlainLaunch& L)
 {
     const bool flat = L.cols.table_flat != 0u;
-    if(L.profile) return LOOM_B200_OK;
-    unsigned& blk = h->plain_blk[flat];
+    unsigned&  blk = h->plain_blk[flat];
     if(blk == 0)
     {
         int regs = 0;
