@@ -488,6 +488,15 @@ launch_graph(loom_b200_handle* h, const RegroupLaunch& L, uint64_t admit, cudaSt
     return LOOM_B200_OK;
 }
 
+/// Whether a grid can have the CTAs that n threads need.
+constexpr bool
+fits_grid(const unsigned long long n, const unsigned long long block)
+{
+    return (n + block - 1u) / block <= 0x7fffffffull;
+}
+static_assert(fits_grid(32ull * 0x7fffffff, 32) && !fits_grid(32ull * 0x7fffffff + 1, 32));
+static_assert(fits_grid(32ull * 0x7fffffff + 1, kDefaultPlainBlock));
+
 /// CTA size of a plain launch whose caller named none: the default, or one
 /// warp for a kernel of so many registers (kOneWarpRegs) that the 32 CTAs an
 /// SM can hold are as many warps as its registers can.  The registers of a
@@ -498,7 +507,9 @@ launch_graph(loom_b200_handle* h, const RegroupLaunch& L, uint64_t admit, cudaSt
 /// -> 32 us) as half their warps do not fit.  Profiled launches take the size
 /// of the launch they describe (by the unprofiled kernel's registers); of the
 /// several Loom threads per CUDA thread of loop-free programs they run one,
-/// which puts the same threads together in a warp.
+/// which puts the same threads together in a warp.  A launch whose CTAs of one
+/// warp would exceed a grid runs the default size, which takes eight times as
+/// many threads.
 int
 plain_block(loom_b200_handle* h, PlainLaunch& L)
 {
@@ -511,8 +522,8 @@ plain_block(loom_b200_handle* h, PlainLaunch& L)
         LB_CUDA(h->e->plain_attrs(false, flat, 1u, &regs, &max));
         blk = regs >= kOneWarpRegs ? 32u : kDefaultPlainBlock;
     }
-    L.block = blk;
-    if(blk == 32u && h->e->spread)
+    L.block = fits_grid(L.n, blk) ? blk : kDefaultPlainBlock;
+    if(L.block == 32u && h->e->spread)
     {
         const unsigned long long warps = static_cast<unsigned long long>(h->sms) * kSpreadWarps;
         while(L.lanes > 1u && L.n <= L.lanes / 2u * warps) L.lanes /= 2u;
