@@ -103,11 +103,13 @@ typedef struct loom_b200_opts
                              admits every input at once and needs no queue
                              state (a few KB instead of 2 x row bytes per
                              thread in flight) */
-    uint32_t burst;       /* regroup: blocks a lane runs between two votes
-                             (schedules 0 and 1 without the cost model, in
-                             programs of several loops: fewer once 8 lanes
-                             have halted and there are inputs for them; the
-                             period is charged the whole burst) */
+    uint32_t burst;       /* regroup: blocks a lane runs between two votes.
+                             Schedules 0 and 1 without the cost model, in
+                             programs of several loops: its visits of loop
+                             headers, a loop on one block (up to 1024
+                             iterations) one visit; the burst ends once 8
+                             lanes have halted and there are inputs for
+                             them.  `period` counts iterations there too */
     uint32_t spread_lanes; /* regroup: when the majority block holds at least
                               this many lanes, every live lane runs the
                               burst (33 = majority lanes only) */

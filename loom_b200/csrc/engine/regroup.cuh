@@ -79,7 +79,7 @@ struct RegroupParams
     unsigned            cap;      // population: entries per queue, multiple of 32
     unsigned            utr;      // majority quorum, lanes
     unsigned            period;   // block steps per tile per round (LOOM_B200_PERIOD_UNBOUNDED: none)
-    unsigned            burst;    // blocks a lane runs between two votes
+    unsigned            burst;    // blocks a lane runs between two votes (kOrdered: visits of loop headers)
     unsigned            spread;   // majority size from which all live lanes run
     unsigned            prefetch; // prefetch the next input of every lane
     unsigned            refill;   // halted lanes claim new inputs at once
@@ -455,16 +455,18 @@ regroup_kernel(const RegroupParams p)
                 // of the chosen group `burst` visits; in programs of several
                 // loops the lanes take them in that same order (kOrdered)
                 // instead of each along its own path: a 320x240x16 render
-                // with default options 2.25 -> 1.10 ms (0.99 ms with loops
-                // run to their end within one visit, but then neither burst
-                // nor period bounds what a tile runs in a round).
-                unsigned visits = kOrdered && pc >= 0 && (mc >= p.spread || pc == m) ? p.burst : 0u;
+                // with default options 2.25 -> 1.03 ms (0.99 ms with the
+                // iterations of a loop on one block uncounted, but then the
+                // period does not bound what a tile runs in a round; 1.10 ms
+                // with iterations taken off the burst's visits).
+                unsigned visits = pc >= 0 && (mc >= p.spread || pc == m) ? p.burst : 0u;
+                unsigned left   = p.period - steps; // of the lane's steps in this round
                 for(unsigned i = 0; kOrdered || i < (minpc ? p.burst : 1u); ++i)
                 {
                     bool run;
                     if(kOrdered)
                     {
-                        const unsigned rk = pc >= 0 && visits ? s_rank[pc] : 0xffffffffu;
+                        const unsigned rk = pc >= 0 && visits && left ? s_rank[pc] : 0xffffffffu;
                         const unsigned lo = __reduce_min_sync(FULL, rk);
                         if(lo == 0xffffffffu) break;
                         run = rk == lo;
@@ -498,11 +500,17 @@ regroup_kernel(const RegroupParams p)
                         run = pc >= 0 && (p.schedule == 3u || mc >= p.spread || pc == m);
                     if constexpr(kOrdered)
                     {
-                        // a lane may spend what it has left of the burst on
-                        // one loop; iterations count as visits do
-                        unsigned spin = visits;
-                        if(run) pc = K::template run_steps<kProf, kFlat, false>(pc, R, ctx, 1u, false, spin);
-                        if(run) visits = spin < visits ? spin : visits - 1u;
+                        // a visit is charged as one step, and as one for
+                        // each iteration of a loop on one block
+                        if(run)
+                        {
+                            --visits;
+                            --left;
+                            const unsigned given = left < kSelfLoopSpin ? left : kSelfLoopSpin;
+                            unsigned       spin  = given;
+                            pc = K::template run_steps<kProf, kFlat, false>(pc, R, ctx, 1u, false, spin);
+                            left -= given - spin;
+                        }
                     }
                     else if(run)
                     {
@@ -534,10 +542,10 @@ regroup_kernel(const RegroupParams p)
                        static_cast<unsigned>(__popc(__ballot_sync(FULL, pc == kHalt))) >= p.refill_lanes)
                         break;
                 }
-                // a burst that ended early counts in full: `period` is the
-                // most a tile runs in a round (what its lanes ran, summed
-                // exactly: 320x240x16 with default options 1.10 -> 1.12 ms)
-                if(kPark && p.period != LOOM_B200_PERIOD_UNBOUNDED) steps += p.burst;
+                if constexpr(kOrdered)
+                    steps = p.period - __reduce_min_sync(FULL, left);
+                else if(kPark && p.period != LOOM_B200_PERIOD_UNBOUNDED)
+                    steps += p.burst;
                 const unsigned hm = __ballot_sync(FULL, pc == kHalt);
                 if(hm != 0u)
                 {
