@@ -49,10 +49,12 @@ from __future__ import annotations
 
 import argparse
 import concurrent.futures
+import hashlib
 import json
 import math
 import os
 import pathlib
+import re
 import statistics
 import subprocess
 import sys
@@ -671,13 +673,25 @@ def same_bits(got, want, kernel: str = "") -> bool:
 
 
 # ---------------------------------------------------------------- GPU arm
+def code_digest(kernel: str) -> str:
+    """Digest of the device code behind a kernel's regrouping launches: its
+    generated source and the engine's headers, without comments and layout."""
+    h = hashlib.sha256()
+    src = ROOT / "loom_b200" / "csrc"
+    for f in (src / "gen" / f"{kernel}.cu", src / "engine" / "common.cuh", src / "engine" / "regroup.cuh"):
+        text = re.sub(r"//[^\n]*|/\*.*?\*/", "", f.read_text(), flags=re.S)
+        h.update("".join(text.split()).encode())
+    return h.hexdigest()[:16]
+
+
 def ncu_rooflines(w, kern_ms: float, sm_mhz: float, path: pathlib.Path = None):
     """Figures of the dominant kernel that come from an ncu capture
     (profiles/roofline_traffic.json, per thread, scaled to this launch):
     DRAM traffic per launch, and the issue roofline — SASS warp instructions
     per second against one per cycle on each of the 148 x 4 SM
     sub-partitions at `sm_mhz`.  The issue figure is given only when the
-    capture was taken with the same regrouping options.  Returns (traffic
+    capture was taken with the same regrouping options, and says whether it
+    was taken with the present code.  Returns (traffic
     bytes or None, issue dict or None)."""
     tf = path or ROOT / "profiles" / "roofline_traffic.json"
     if not tf.exists():
@@ -696,6 +710,7 @@ def ncu_rooflines(w, kern_ms: float, sm_mhz: float, path: pathlib.Path = None):
             "unit": "G warp instructions/s",
             "frac": round(got / top, 4),
             "sass_warp_inst_per_thread": t["sass_warp_inst_per_thread"],
+            "capture_of_this_code": t.get("code") == code_digest(w.kernel),
         }
     return traffic, issue
 
