@@ -231,8 +231,9 @@ typedef struct loom_b200_launch
     uint32_t               num_instances;
     uint32_t               pad;
     const uint32_t*        table;           /* or NULL */
-    uint64_t               table_words;     /* device launches: 0 = unstated (the
-                                               allocation then bounds it) */
+    uint64_t               table_words;     /* device launches: 0 = unstated (its
+                                               allocation, or the reservation
+                                               it is mapped in, bounds it) */
 } loom_b200_launch;
 
 typedef struct loom_b200_handle loom_b200_handle;

@@ -25,21 +25,27 @@ loom_b200::table_flat(const void* table, const unsigned long long words)
 {
     if(!table) return true;
     if(words) return words <= kFlatWords;
-    using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
-    static const Range range = []() -> Range
+    // The address range that the pointer belongs to: an allocation, or the
+    // whole reservation where memory is mapped piece by piece into one (the
+    // allocation that cuMemGetAddressRange names is then a piece, which does
+    // not bound the table).
+    using Attribute = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const Attribute attribute = []() -> Attribute
     {
         void*                           fn = nullptr;
         cudaDriverEntryPointQueryResult q  = cudaDriverEntryPointSymbolNotFound;
-        if(cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+        if(cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &q) != cudaSuccess ||
            q != cudaDriverEntryPointSuccess)
             fn = nullptr;
         cudaGetLastError();
-        return reinterpret_cast<Range>(fn);
+        return reinterpret_cast<Attribute>(fn);
     }();
     CUdeviceptr       base = 0;
     size_t            size = 0;
     const CUdeviceptr at   = reinterpret_cast<CUdeviceptr>(table);
-    if(!range || range(&base, &size, at) != CUDA_SUCCESS) return false;
+    if(!attribute || attribute(&base, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
+       attribute(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS)
+        return false;
     return (base + size - at) / sizeof(uint32_t) <= kFlatWords;
 }
 
